@@ -45,7 +45,7 @@ struct KernelArgs {
     int32_t ny, nx;
     int32_t adu;            // 1: data are ADU, convert (ADU - offset) * gain
     int32_t iterations;
-    int32_t tpr;            // threads per ROI: 1, 2, 4, 8, 16 or 32
+    int32_t tpr;            // threads per ROI: 1, 2, 4, 8 or 32
     float sqrt2pi;          // sqrt(2f * Float32(pi)) as Julia evaluates it
     float psf[8];
     float lower[6], upper[6], max_step[6];
@@ -288,47 +288,40 @@ __device__ __forceinline__ void walk_entry(int t, const Axis &a, EdgeWalk &w, fl
     w.fa = fa;
 }
 
-// Astigmatic width model, src/psf_derivatives.jl:118-163 (per iteration, scalar).
+// Astigmatic width model, src/psf_derivatives.jl:118-163 (per iteration, scalar):
+// one axis' width and its first and second derivatives with respect to z
+// (off: -gamma for x, +gamma for y).
+__device__ __forceinline__ void astig_width(float z, float off, float s0, float A, float B, float d,
+                                            float &s, float &ds, float &d2s)
+{
+    const float zd = __fdiv_rn(__fadd_rn(z, off), d);
+    const float zd2 = __fmul_rn(zd, zd);
+    const float zd3 = __fmul_rn(zd2, zd);
+    const float al = __fadd_rn(__fadd_rn(__fadd_rn(1.0f, zd2), __fmul_rn(A, zd3)),
+                               __fmul_rn(B, jl_pow4f(zd)));
+    const float ra = sqrtf(al);
+    s = __fmul_rn(s0, ra);
+    const float da = __fdiv_rn(__fadd_rn(__fadd_rn(__fmul_rn(2.0f, zd), __fmul_rn(__fmul_rn(3.0f, A), zd2)),
+                                         __fmul_rn(__fmul_rn(4.0f, B), zd3)), d);
+    const float h = __fdiv_rn(s0, __fmul_rn(2.0f, ra));
+    ds = __fmul_rn(h, da);
+    const float d2a = __fdiv_rn(__fadd_rn(__fadd_rn(2.0f, __fmul_rn(__fmul_rn(6.0f, A), zd)),
+                                          __fmul_rn(__fmul_rn(12.0f, B), zd2)), __fmul_rn(d, d));
+    // alpha^1.5f0 (Julia rounds a Float64 pow once); alpha*sqrt(alpha) in FP32 is
+    // within 1.5 ulp and avoids an FP64 pow per iteration.
+    const float p15 = __fmul_rn(al, ra);
+    d2s = __fadd_rn(__fmul_rn(-__fdiv_rn(s0, __fmul_rn(4.0f, p15)), __fmul_rn(da, da)),
+                    __fmul_rn(h, d2a));
+}
+
 struct AstigWidths {
     float sx, sy, dsx, dsy, d2sx, d2sy;
 };
 
 __device__ __forceinline__ void astig_widths(float z, const float *psf, AstigWidths &w)
 {
-    const float sx0 = psf[0], sy0 = psf[1], Ax = psf[2], Ay = psf[3], Bx = psf[4], By = psf[5];
-    const float gam = psf[6], d = psf[7];
-    const float zdx = __fdiv_rn(__fadd_rn(z, -gam), d);
-    const float zdy = __fdiv_rn(__fadd_rn(z, gam), d);
-    const float zdx2 = __fmul_rn(zdx, zdx), zdy2 = __fmul_rn(zdy, zdy);
-    const float zdx3 = __fmul_rn(zdx2, zdx), zdy3 = __fmul_rn(zdy2, zdy);
-    const float ax = __fadd_rn(__fadd_rn(__fadd_rn(1.0f, zdx2), __fmul_rn(Ax, zdx3)),
-                               __fmul_rn(Bx, jl_pow4f(zdx)));
-    const float ay = __fadd_rn(__fadd_rn(__fadd_rn(1.0f, zdy2), __fmul_rn(Ay, zdy3)),
-                               __fmul_rn(By, jl_pow4f(zdy)));
-    const float rax = sqrtf(ax), ray = sqrtf(ay);
-    w.sx = __fmul_rn(sx0, rax);
-    w.sy = __fmul_rn(sy0, ray);
-    const float dax = __fdiv_rn(__fadd_rn(__fadd_rn(__fmul_rn(2.0f, zdx), __fmul_rn(__fmul_rn(3.0f, Ax), zdx2)),
-                                          __fmul_rn(__fmul_rn(4.0f, Bx), zdx3)), d);
-    const float day = __fdiv_rn(__fadd_rn(__fadd_rn(__fmul_rn(2.0f, zdy), __fmul_rn(__fmul_rn(3.0f, Ay), zdy2)),
-                                          __fmul_rn(__fmul_rn(4.0f, By), zdy3)), d);
-    const float hx = __fdiv_rn(sx0, __fmul_rn(2.0f, rax));
-    const float hy = __fdiv_rn(sy0, __fmul_rn(2.0f, ray));
-    w.dsx = __fmul_rn(hx, dax);
-    w.dsy = __fmul_rn(hy, day);
-    const float dd = __fmul_rn(d, d);
-    const float d2ax = __fdiv_rn(__fadd_rn(__fadd_rn(2.0f, __fmul_rn(__fmul_rn(6.0f, Ax), zdx)),
-                                           __fmul_rn(__fmul_rn(12.0f, Bx), zdx2)), dd);
-    const float d2ay = __fdiv_rn(__fadd_rn(__fadd_rn(2.0f, __fmul_rn(__fmul_rn(6.0f, Ay), zdy)),
-                                           __fmul_rn(__fmul_rn(12.0f, By), zdy2)), dd);
-    // alpha^1.5f0 (Julia rounds a Float64 pow once); alpha*sqrt(alpha) in FP32 is
-    // within 1.5 ulp and avoids an FP64 pow per iteration.
-    const float p15x = __fmul_rn(ax, rax);
-    const float p15y = __fmul_rn(ay, ray);
-    w.d2sx = __fadd_rn(__fmul_rn(-__fdiv_rn(sx0, __fmul_rn(4.0f, p15x)), __fmul_rn(dax, dax)),
-                       __fmul_rn(hx, d2ax));
-    w.d2sy = __fadd_rn(__fmul_rn(-__fdiv_rn(sy0, __fmul_rn(4.0f, p15y)), __fmul_rn(day, day)),
-                       __fmul_rn(hy, d2ay));
+    astig_width(z, -psf[6], psf[0], psf[2], psf[4], psf[7], w.sx, w.dsx, w.d2sx);
+    astig_width(z, psf[6], psf[1], psf[3], psf[5], psf[7], w.sy, w.dsy, w.d2sy);
 }
 
 // ---- group reductions --------------------------------------------------------

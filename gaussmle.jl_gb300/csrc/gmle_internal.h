@@ -11,8 +11,8 @@
 #include <vector>
 
 #include "../../include/gaussmle_gb300.h"
-#include "gmle_generic.h"
 #include "gmle_launch.cuh"
+#include "gmle_warp.h"
 
 namespace gmle_rt {
 

@@ -19,8 +19,8 @@ namespace gmle {
 
 // Box sizes with a compiled specialisation: every edge length 3..16 (the
 // configurations use 7..15; the reference accepts any box >= 3,
-// src/interface.jl:22).  Larger boxes run in the runtime-box kernel
-// (gmle_fit_generic.cu).
+// src/interface.jl:22).  Larger boxes run with one warp per ROI
+// (gmle_fit_warp.cu).
 constexpr int kMinBox = 3, kMaxBox = 16;
 constexpr int kNumBoxes = kMaxBox - kMinBox + 1;
 

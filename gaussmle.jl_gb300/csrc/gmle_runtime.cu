@@ -55,10 +55,10 @@ gmle_status check_desc(gmle_ctx *ctx, const gmle_fit_desc *d)
     if (!d) return fail(ctx, GMLE_INVALID_ARG, "desc is NULL");
     if (d->model < 0 || d->model > 3)
         return fail(ctx, GMLE_UNSUPPORTED_MODEL, "unknown model id %d", d->model);
-    if (!gmle::box_supported(d->box) && !gmle::generic_box(d->box))
+    if (!gmle::box_supported(d->box) && !gmle::large_box(d->box))
         return fail(ctx, GMLE_UNSUPPORTED_BOX, "box size %d: ROIs of %d..%d pixels are supported",
-                    d->box, gmle::kMinBox, gmle::kGenericMaxBox);
-    if (gmle::generic_box(d->box) && d->method != GMLE_METHOD_NEWTON)
+                    d->box, gmle::kMinBox, gmle::kLargeMaxBox);
+    if (gmle::large_box(d->box) && d->method != GMLE_METHOD_NEWTON)
         return fail(ctx, GMLE_UNSUPPORTED_BOX,
                     "box size %d: the full-Hessian method takes boxes %d..%d", d->box,
                     gmle::kMinBox, gmle::kMaxBox);
@@ -109,7 +109,7 @@ namespace gmle_rt {
 Tuning pick_tuning(gmle_ctx *ctx, const gmle_fit_desc *d, int64_t n)
 {
     const bool scmos = d->camera != GMLE_CAMERA_POISSON;
-    if (gmle::generic_box(d->box)) return {1, gmle::generic_rois_per_block(d->box, scmos)};
+    if (gmle::large_box(d->box)) return {32, gmle::warp_rois_per_block(d->box, scmos)};
     auto it = ctx->tuning.find({d->model, d->box, (int)scmos});
     Tuning t = it != ctx->tuning.end() ? it->second
                                        : default_tuning(ctx->num_sms, d->model, d->box, scmos, n);
@@ -163,7 +163,7 @@ cudaError_t launch(gmle_ctx *ctx, const gmle_fit_desc *d, const KernelArgs &a, i
 {
     const bool scmos = d->camera != GMLE_CAMERA_POISSON;
     ctx->launches++;
-    if (gmle::generic_box(d->box)) return gmle::launch_fit_generic(d->model, d->box, scmos, a, s);
+    if (a.tpr == 32) return gmle::launch_fit_warp(d->model, d->box, scmos, a, rpb, s);
     gmle::LaunchShape shape{a.tpr, rpb, 0};
     shape.lm = d->method == GMLE_METHOD_FISHER_LM;
     return gmle::launch_fit(d->model, d->box, scmos, a, gmle::TileTable{}, shape, s);
@@ -547,14 +547,14 @@ gmle_status gmle_autotune(gmle_ctx *ctx, const gmle_fit_desc *desc, const float 
         return fail(ctx, GMLE_INVALID_ARG, "sCMOS fit needs ROI corners");
     cudaSetDevice(ctx->device);
     const bool scmos = desc->camera != GMLE_CAMERA_POISSON;
-    if (gmle::generic_box(desc->box)) {
-        // one launch shape: the run-time-box kernel's
+    if (gmle::large_box(desc->box)) {
+        // one launch shape: one warp per ROI
         const Tuning t = pick_tuning(ctx, desc, n);
         cudaEvent_t e0, e1;
         CK(cudaEventCreate(&e0), "cudaEventCreate");
         CK(cudaEventCreate(&e1), "cudaEventCreate");
         KernelArgs a = make_args(ctx, desc, d_data, d_x_corners, d_y_corners, n, d_params,
-                                 d_crlb, d_llr, d_flags, 1);
+                                 d_crlb, d_llr, d_flags, t.tpr);
         cudaError_t e = cudaEventRecord(e0, ctx->s_fit);
         if (e == cudaSuccess) e = launch(ctx, desc, a, t.rois_per_block, ctx->s_fit);
         if (e == cudaSuccess) e = cudaEventRecord(e1, ctx->s_fit);
@@ -564,7 +564,7 @@ gmle_status gmle_autotune(gmle_ctx *ctx, const gmle_fit_desc *desc, const float 
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "autotune launch");
-        if (threads_per_roi) *threads_per_roi = 1;
+        if (threads_per_roi) *threads_per_roi = t.tpr;
         if (rois_per_block) *rois_per_block = t.rois_per_block;
         if (ms_per_fit) *ms_per_fit = ms;
         return GMLE_OK;

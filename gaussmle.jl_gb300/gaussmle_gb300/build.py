@@ -3,7 +3,8 @@
 The library is the product: the fit kernels, compiled from one family source
 (csrc/gmle_fit_family.cu) as 24 units - per PSF model (4), camera family (2)
 and part (3: one thread per ROI for the odd boxes 5..15, for the other boxes
-3..16, several lanes per ROI) - plus the runtime-box kernel and the C-ABI
+3..16, several lanes per ROI) - the fit with one warp per ROI
+(csrc/gmle_fit_warp.cu) as 8 units per model and camera family, and the C-ABI
 runtime, compiled in parallel (one -gencode, no cmake; the heaviest units
 first) and linked into ``<package root>/lib/libgaussmle_sm100a.so``.
 """
@@ -33,8 +34,10 @@ _NAMES = {0: "xynb", 1: "xynbs", 2: "xynbsxsy", 3: "astig"}
 UNITS = [(FAMILY, f"gmle_fit_{_NAMES[m]}_{'scmos' if c else 'poisson'}_p{p}",
           [f"-DGMLE_MODEL={m}", f"-DGMLE_SCMOS={c}", f"-DGMLE_PART={p}"])
          for p in (0, 1, 2) for m in (3, 2, 1, 0) for c in (1, 0)] + \
+        [("gmle_fit_warp.cu", f"gmle_fit_warp_{_NAMES[m]}_{'scmos' if c else 'poisson'}",
+          [f"-DGMLE_MODEL={m}", f"-DGMLE_SCMOS={c}"]) for m in (3, 2, 1, 0) for c in (1, 0)] + \
         [(src, Path(src).stem, []) for src in
-         ("gmle_fit_generic.cu", "gmle_runtime.cu", "gmle_server.cu", "gmle_noalloc.cu",
+         ("gmle_runtime.cu", "gmle_server.cu", "gmle_noalloc.cu",
           "gmle_pvalue.cu", "gmle_frames.cu", "gmle_simulate.cu", "gmle_math.cu")]
 
 
