@@ -148,12 +148,15 @@ int nparams(int model);
 gmle_status init_mixed_set(gmle_ctx *ctx, MixedSet &m);
 void free_mixed_set(MixedSet &m);
 // How a table launch picks its shape: from the context's tuning for the
-// kind, else the size-based default for `shape_rois` ROIs (0: the kind's ROIs
-// in this submission).  Persistent grids are full (SMs x resident blocks)
+// kind, else the size-based default for a submission of `shape_rois` ROIs (0:
+// this one's), with `line` ROIs per SM from which one thread fits a ROI
+// (default_tuning).  Persistent grids are full (SMs x resident blocks)
 // when `full_grid`, else no larger than the tiles.
+constexpr int kPlainLine = 80, kServingLine = 80, kSubmissionLine = 200;
 struct PlanOptions {
     bool allow_plain = true;
     int64_t shape_rois = 0;
+    int line = kSubmissionLine;
     // persistent table launches (a grid of resident blocks that take tiles from
     // a counter; full_grid: sized for the GPU whatever the tiles) or one block
     // per tile
@@ -180,8 +183,10 @@ gmle_status enqueue_table_launch(gmle_ctx *ctx, MixedSet &m, const TableLaunch &
 // m.fork when there are several, joined back into s.
 gmle_status enqueue_plan(gmle_ctx *ctx, MixedSet &m, const MixedPlan &plan, cudaStream_t s);
 gmle_status validate_groups(gmle_ctx *ctx, const gmle_group *groups, int32_t ngroups);
-Tuning pick_tuning(gmle_ctx *ctx, const gmle_fit_desc *d, int64_t n);
-Tuning default_tuning(int num_sms, int model, int box, bool scmos, int64_t n);
+Tuning pick_tuning(gmle_ctx *ctx, const gmle_fit_desc *d, int64_t n, int64_t together = 0,
+                   int line = kPlainLine);
+Tuning default_tuning(int num_sms, int model, int box, bool scmos, int64_t n, int64_t together = 0,
+                      int line = kPlainLine);
 gmle::KernelArgs make_args(gmle_ctx *ctx, const gmle_fit_desc *d, const float *data,
                            const int32_t *xc, const int32_t *yc, int64_t n, float *params,
                            float *crlb, float *llr, uint8_t *flags, int tpr);

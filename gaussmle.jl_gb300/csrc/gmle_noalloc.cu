@@ -213,6 +213,8 @@ extern "C" gmle_status gmle_fit_mixed_device_noalloc(const gmle_group *groups, i
     KernelArgs *h_args = reinterpret_cast<KernelArgs *>(g_stage + kArgsOff);
     unsigned long long *d_counters = reinterpret_cast<unsigned long long *>(S.scratch + kCountersOff);
     int used = 0;
+    int64_t together = 0;
+    for (int k = 0; k < ngroups; k++) together += std::max<int64_t>(groups[k].n, 0);
     int first[kKinds] = {};
     gmle::LaunchShape shape[kKinds] = {};
     for (int kind = 0; kind < kKinds; kind++) {
@@ -227,7 +229,8 @@ extern "C" gmle_status gmle_fit_mixed_device_noalloc(const gmle_group *groups, i
         if (cnt == 0) continue;
         const gmle_fit_desc &d0 = groups[g_order[0]].desc;
         const bool scmos = d0.camera != GMLE_CAMERA_POISSON;
-        const gmle_rt::Tuning t = gmle_rt::default_tuning(S.num_sms, d0.model, d0.box, scmos, rois);
+        const gmle_rt::Tuning t = gmle_rt::default_tuning(S.num_sms, d0.model, d0.box, scmos, rois,
+                                                             together, gmle_rt::kSubmissionLine);
         int64_t tiles = 0;
         for (int q = 0; q < cnt; q++) {
             const gmle_group &G = groups[g_order[q]];

@@ -83,36 +83,59 @@ gmle_status check_desc(gmle_ctx *ctx, const gmle_fit_desc *d)
 
 namespace gmle_rt {
 
-// Launch shape: enough threads to fill the GPU (threads per ROI grows for small
-// batches), and ROIs per block bounded by shared memory.
-Tuning default_tuning(int num_sms, int model, int box, bool scmos, int64_t n)
+// Launch shape when none is tuned, from the batch's size.
+//
+// One thread per ROI does the least work per ROI and wins as soon as the batch
+// gives every SM a few warps; several lanes per ROI shorten a fit's chain of
+// dependent passes when it does not.  Measured over models, boxes 5..16 and
+// cameras (us, 4 lanes / one thread): 5 000 ROIs XYNB 11x11 57 / 78, astigmatic
+// 15x15 115 / 131; 10 000: XYNB 11x11 70 / 78, 11x11 sCMOS 74 / 70, XYNBS 13x13
+// sCMOS 115 / 104; 20 000: XYNB 11x11 121 / 98, XYNBS 13x13 sCMOS 205 / 148;
+// 300 000: 1208 / 610 and 2295 / 1112.  The line is drawn at 80 ROIs per SM.
+//
+// `together` > 0: the launch is one of several, of `together` ROIs in all, that
+// share the SMs.  A submission that waits for its slowest launch (`line` 200 ROIs
+// per SM) gains from short chains for longer than serving steps that overlap
+// (80).  Measured on the five kinds of the sCMOS mixed batch (us, 4 lanes / one
+// thread): 12 000 ROIs 187 / 295, 25 000 246 / 294, 50 000 421 / 313; served
+// requests of 12 000 ROIs 387 / 394, 25 000 461 / 394, 100 000 968 / 774.
+//
+// ROIs per block of the one-thread kernel: with sCMOS data 128, whose four warps
+// use their tensor-memory columns fully; Poisson data the block that lets
+// the shared memory hold most ROIs (astigmatic 15x15, 300 000 ROIs: 1428 us in
+// blocks of 128, two of which fit an SM, 1668 us in blocks of 64, three of
+// which fit).  Below 256 ROIs per SM smaller blocks spread over the SMs evenly
+// (20 000 XYNB 11x11 ROIs: 98 us in blocks of 32; 40 000 11x11 sCMOS: 131 us in
+// blocks of 96, 137 us of 128).
+Tuning default_tuning(int num_sms, int model, int box, bool scmos, int64_t n, int64_t together,
+                      int line)
 {
-    // Resident ROIs per SM are bounded by shared memory; threads per ROI grow
-    // until about 16 warps per SM are resident and the batch fills the GPU.
-    const size_t per_roi = gmle::smem_bytes(model, box, scmos, 1, 1);
-    const int64_t rois_per_sm = (int64_t)((200 * 1024) / per_roi);
-    const int64_t want_threads_sm = 512;
-    int tpr = 1;
-    if (rois_per_sm < want_threads_sm || n < (int64_t)num_sms * want_threads_sm) tpr = 4;
-    // one thread per ROI with sCMOS data: blocks of 4 warps use the tensor
-    // memory that holds the variance tiles fully
-    int rpb = tpr == 1 ? (scmos ? 128 : 32) : 128 / tpr;
-    while (rpb * tpr > 32 && gmle::smem_bytes(model, box, scmos, tpr, rpb) > 100 * 1024) rpb /= 2;
-    if (rpb * tpr < 32) rpb = 32 / tpr;
-    return {tpr, rpb};
+    if ((together > 0 ? together : n) < (int64_t)line * num_sms) return {4, 32};
+    const bool spread = together == 0 && n < (int64_t)256 * num_sms;
+    if (scmos) return {1, spread ? 96 : 128};
+    if (spread) return {1, 32};
+    int best = 64, most = 0;
+    for (int rpb : {64, 128, 32}) {
+        // a block takes 1 KiB beside its own shared memory of the SM's 228 KiB
+        const size_t block = gmle::smem_bytes(model, box, scmos, 1, rpb) + 1024;
+        const int rois = rpb * (int)(228 * 1024 / block);
+        if (rois > most) { most = rois; best = rpb; }
+    }
+    return {1, best};
 }
 
 }  // namespace gmle_rt
 
 namespace gmle_rt {
 
-Tuning pick_tuning(gmle_ctx *ctx, const gmle_fit_desc *d, int64_t n)
+Tuning pick_tuning(gmle_ctx *ctx, const gmle_fit_desc *d, int64_t n, int64_t together, int line)
 {
     const bool scmos = d->camera != GMLE_CAMERA_POISSON;
     if (gmle::large_box(d->box)) return {32, gmle::warp_rois_per_block(d->box, scmos)};
     auto it = ctx->tuning.find({d->model, d->box, (int)scmos});
     Tuning t = it != ctx->tuning.end() ? it->second
-                                       : default_tuning(ctx->num_sms, d->model, d->box, scmos, n);
+                                       : default_tuning(ctx->num_sms, d->model, d->box, scmos, n,
+                                                        together, line);
     if (d->method == GMLE_METHOD_FISHER_LM && t.tpr != 1) {
         // the full-Hessian method runs one thread per ROI; 128-thread blocks
         // use the tensor memory of sCMOS variance tiles fully
@@ -739,10 +762,11 @@ gmle_status plan_mixed(gmle_ctx *ctx, const gmle_group *groups, int32_t ngroups,
     plan = MixedPlan();
     m.pool_used = 0;
     std::vector<int> by_kind[kKinds];
-    int64_t rois[kKinds] = {};
+    int64_t rois[kKinds] = {}, together = 0;
     for (int k = 0; k < ngroups; k++) {
         const gmle_group &G = groups[k];
         if (G.n <= 0) continue;
+        together += G.n;
         if (opt.allow_plain && G.n >= kPlainGroupRois) {
             plan.plain.push_back(G);
             continue;
@@ -759,7 +783,8 @@ gmle_status plan_mixed(gmle_ctx *ctx, const gmle_group *groups, int32_t ngroups,
         L.model = d0.model;
         L.box = d0.box;
         L.scmos = d0.camera != GMLE_CAMERA_POISSON;
-        const Tuning t = pick_tuning(ctx, &d0, opt.shape_rois > 0 ? opt.shape_rois : rois[kind]);
+        const Tuning t = pick_tuning(ctx, &d0, rois[kind],
+                                     opt.shape_rois > 0 ? opt.shape_rois : together, opt.line);
         const int rpb = t.rois_per_block;
         int64_t tiles = 0;
         for (int k : by_kind[kind]) tiles += (groups[k].n + rpb - 1) / rpb;
@@ -912,7 +937,9 @@ extern "C" gmle_status gmle_fit_mixed_device(gmle_ctx *ctx, const gmle_group *gr
     gmle_status st = init_mixed_set(ctx, ctx->mixed);
     if (st != GMLE_OK) return st;
     MixedPlan plan;
-    st = plan_mixed(ctx, groups, ngroups, ctx->mixed, plan, PlanOptions());
+    PlanOptions opt;
+    opt.persistent = false;  // one block per tile: the launches interleave on the SMs
+    st = plan_mixed(ctx, groups, ngroups, ctx->mixed, plan, opt);
     if (st != GMLE_OK) return st;
     st = upload_plan(ctx, ctx->mixed, plan, (cudaStream_t)stream, true);
     if (st != GMLE_OK) return st;

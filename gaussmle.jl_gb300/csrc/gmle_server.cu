@@ -371,7 +371,8 @@ struct Server {
         std::lock_guard<std::mutex> lk(ctx->mu);
         PlanOptions opt;
         opt.allow_plain = false;
-        opt.shape_rois = cfg.max_step_rois;
+        opt.shape_rois = cfg.use_graphs ? cfg.max_step_rois : 0;
+        opt.line = kServingLine;
         // a graph replays a fixed grid: persistent launches; direct launches
         // take one block per tile
         opt.persistent = cfg.use_graphs != 0;
