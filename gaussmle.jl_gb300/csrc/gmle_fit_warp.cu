@@ -4,15 +4,17 @@
 // -DGMLE_SCMOS=0|1.
 //
 // It fits the ROIs beyond 16 pixels (17..64), whose pixels and tables exceed
-// what one thread can hold.
+// what one thread can hold, and small batches of the smaller boxes, whose time is
+// the latency of a fit's dependent passes (default_tuning draws the line).
 //
 // A warp's lanes are a grid of 8 column by 4 row classes: lane (rx, ry) owns
 // the pixels of columns rx, rx + 8, ... and rows ry, ry + 4, ..., at most
 // RMAX rows.  Up to 32 pixels per lane (boxes to 32) stay in its registers for
 // the whole fit; larger boxes read them from shared memory.  Per pass:
 //  * lanes 0-15 set up the x axis, lanes 16-31 the y axis;
-//  * every lane evaluates one pixel edge (one erf, one exp); table entries are
-//    differences with the neighbouring lane's, written to shared memory;
+//  * every lane evaluates one pixel edge (one erf, one exp; up to 15 pixels both
+//    axes at once); table entries are differences with the neighbouring lane's,
+//    written to shared memory;
 //  * every lane sums its pixels and applies the column and row terms, which
 //    are linear in those sums, to its partial sums;
 //  * the P (gradient, Hessian) pairs are summed and scattered over the lanes,
@@ -27,7 +29,7 @@
 // 21x21 sCMOS), the latency of a pass (no contraction, operands in registers).
 // 12 000 astigmatic 21x21 sCMOS ADU ROIs: 2281 us with one thread per ROI and
 // the pixels and tables in shared memory (one block of 32 threads per SM),
-// 335 us so.
+// 335 us so.  200 XYNB 11x11 ROIs: 45 us with four lanes per ROI, 23 us so.
 #if !defined(GMLE_MODEL) || !defined(GMLE_SCMOS)
 #error "compile with -DGMLE_MODEL=<0..3> -DGMLE_SCMOS=<0|1>"
 #endif
@@ -48,13 +50,16 @@ constexpr int kCols = 8, kRows = 4;  // the lane grid
 template <int RMAX> struct WarpShape {
     static constexpr bool REG = RMAX <= 8;                // pixels in registers
     static constexpr int CMAX = REG ? (RMAX + 1) / 2 : 1;  // columns per lane, in registers
-    static constexpr int RFULL = RMAX == 12 ? 8 : RMAX == 16 ? 12 : RMAX - 1;
+    static constexpr int RFULL = RMAX == 2 ? 0 : RMAX == 12 ? 8 : RMAX == 16 ? 12 : RMAX - 1;
     // columns that lie inside every box of the range (registers only)
-    __host__ __device__ static constexpr int cfull() { return (4 * (RMAX - 1) + 1) / kCols; }
+    __host__ __device__ static constexpr int cfull()
+    {
+        return RMAX == 2 ? 0 : (4 * (RMAX - 1) + 1) / kCols;
+    }
 };
 __host__ __device__ constexpr int rows_per_lane(int box)
 {
-    return box <= 32 ? (box + 3) / 4 : box <= 48 ? 12 : 16;
+    return box <= 8 ? 2 : box <= 32 ? (box + 3) / 4 : box <= 48 ? 12 : 16;
 }
 
 template <int P> struct RoiResult {  // what the inversion needs, per ROI of a block
@@ -180,7 +185,97 @@ __device__ __forceinline__ void warp_entry(int e, const WarpAxis &w, int width, 
     }
 }
 
-// The ROI's start point (src/unified_kernel.jl:158-255) from the lanes' pixels.
+// The start point's parameters from its sums (total, and weighted by column and
+// row; mxx, myy: the astigmatic second moments).
+template <int MODEL>
+__device__ __forceinline__ void warp_start_xy(const int box, float total, float xw, float yw, float &x,
+                                              float &y)
+{
+    const float centre = (float)((box + 1) / 2.0);
+    x = jl_clamp(total > 10.f ? __fdiv_rn(xw, total) : centre, 1.5f, (float)(box - 0.5));
+    y = jl_clamp(total > 10.f ? __fdiv_rn(yw, total) : centre, 1.5f, (float)(box - 0.5));
+}
+template <int MODEL>
+__device__ __forceinline__ void warp_start(float x, float y, float total, float bg, float mxx,
+                                           float myy, const float *psf,
+                                           float (&th)[ModelInfo<MODEL>::P])
+{
+    using S = Slots<MODEL>;
+    th[S::IX] = x;
+    th[S::IY] = y;
+    th[S::IN] = jl_maxf(total, 100.f);
+    th[S::IB] = bg;
+    if (MODEL == 1 || MODEL == 2) th[4] = 1.3f;
+    if (MODEL == 2) th[ModelInfo<MODEL>::P - 1] = 1.3f;
+    if (MODEL == 3) {
+        float z = 0.f;
+        if (total > 10.f) {
+            const float rx = __fdiv_rn(sqrtf(jl_maxf(0.5f, __fdiv_rn(mxx, total))), psf[0]);
+            const float ry = __fdiv_rn(sqrtf(jl_maxf(0.5f, __fdiv_rn(myy, total))), psf[1]);
+            const float da = __fadd_rn(__fmul_rn(rx, rx), -__fmul_rn(ry, ry));
+            z = jl_clamp(__fdiv_rn(__fmul_rn(-da, __fmul_rn(psf[7], psf[7])), __fmul_rn(4.0f, psf[6])),
+                         -600.f, 600.f);
+        }
+        th[2] = z;
+    }
+}
+
+// The ROI's start point (src/unified_kernel.jl:158-255) with every sum in the
+// reference's order (initialize_box), bit for bit.  `scr` holds the ROI's pixels;
+// each lane turns its own into photons above the background, then lanes 0, 1
+// and 2 add the plain, column- and row-weighted sums.
+template <int MODEL, typename Each>
+__device__ __forceinline__ void warp_initialize_exact(const int box, Each each, float *scr, int lane,
+                                                      const float *psf,
+                                                      float (&th)[ModelInfo<MODEL>::P])
+{
+    const int last = box * (box - 1);
+    float edge = 0.f;
+#pragma unroll 4
+    for (int i = 0; i < box; i++) edge = __fadd_rn(edge, scr[i]);
+#pragma unroll 4
+    for (int j = 1; j < box - 1; j++) {
+        edge = __fadd_rn(edge, scr[box * j]);
+        edge = __fadd_rn(edge, scr[box * j + box - 1]);
+    }
+#pragma unroll 4
+    for (int i = 0; i < box; i++) edge = __fadd_rn(edge, scr[last + i]);
+    const float bg = __fdiv_rn(edge, (float)(4 * box - 4));
+    __syncwarp();
+    each([&](int j, int i, float d) { scr[i + box * j] = jl_maxf(0.f, __fadd_rn(d, -bg)); });
+    __syncwarp();
+    // weight 1, column or row (1-based): a + b column + c row
+    const float wc = lane == 1 ? 1.f : 0.f, wr = lane >= 2 ? 1.f : 0.f;
+    const float w0 = lane == 0 ? 1.f : 0.f;
+    float acc = 0.f;
+    for (int j = 0; j < box; j++) {
+        float w = wc * (float)(j + 1) + w0 + wr;  // row 1's weight
+#pragma unroll 4
+        for (int i = 0; i < box; i++) {
+            acc = __fadd_rn(acc, __fmul_rn(scr[i + box * j], w));
+            w += wr;
+        }
+    }
+    const float total = __shfl_sync(0xffffffffu, acc, 0);
+    float x, y, mxx = 0.f, myy = 0.f;
+    warp_start_xy<MODEL>(box, total, __shfl_sync(0xffffffffu, acc, 1),
+                         __shfl_sync(0xffffffffu, acc, 2), x, y);
+    if (MODEL == 3) {  // lane 0: about x, the others: about y
+        acc = 0.f;
+        for (int j = 0; j < box; j++)
+#pragma unroll 4
+            for (int i = 0; i < box; i++) {
+                const float d = lane == 0 ? __fadd_rn((float)(j + 1), -x)
+                                          : __fadd_rn((float)(i + 1), -y);
+                acc = __fadd_rn(acc, __fmul_rn(__fmul_rn(scr[i + box * j], d), d));
+            }
+        mxx = __shfl_sync(0xffffffffu, acc, 0);
+        myy = __shfl_sync(0xffffffffu, acc, 1);
+    }
+    warp_start<MODEL>(x, y, total, bg, mxx, myy, psf, th);
+}
+
+// The ROI's start point from the lanes' pixels, summed over the lanes.
 // each(fn) calls fn(column, row, value) (0-based) for each of the lane's pixels.
 template <int MODEL, typename Each>
 __device__ __forceinline__ void warp_initialize(const int box, Each each, const float *psf,
@@ -201,18 +296,9 @@ __device__ __forceinline__ void warp_initialize(const int box, Each each, const 
     total = warp_sum(total);
     xw = warp_sum(xw);
     yw = warp_sum(yw);
-    const float centre = (float)((box + 1) / 2.0);
-    const float x = jl_clamp(total > 10.f ? __fdiv_rn(xw, total) : centre, 1.5f, (float)(box - 0.5));
-    const float y = jl_clamp(total > 10.f ? __fdiv_rn(yw, total) : centre, 1.5f, (float)(box - 0.5));
-    th[0] = x;
-    th[1] = y;
-    if (MODEL != 3) {
-        th[2] = jl_maxf(total, 100.f);
-        th[3] = bg;
-        if (MODEL >= 1) th[4] = 1.3f;
-        if (MODEL == 2) th[5] = 1.3f;
-    } else {
-        float mxx = 0.f, myy = 0.f;
+    float x, y, mxx = 0.f, myy = 0.f;
+    warp_start_xy<MODEL>(box, total, xw, yw, x, y);
+    if (MODEL == 3) {
         each([&](int j, int i, float d) {
             const float sig = jl_maxf(0.f, d - bg);
             const float dx = (float)(j + 1) - x, dy = (float)(i + 1) - y;
@@ -221,18 +307,8 @@ __device__ __forceinline__ void warp_initialize(const int box, Each each, const 
         });
         mxx = warp_sum(mxx);
         myy = warp_sum(myy);
-        float z = 0.f;
-        if (total > 10.f) {
-            const float rx = __fdiv_rn(sqrtf(jl_maxf(0.5f, __fdiv_rn(mxx, total))), psf[0]);
-            const float ry = __fdiv_rn(sqrtf(jl_maxf(0.5f, __fdiv_rn(myy, total))), psf[1]);
-            const float da = __fadd_rn(__fmul_rn(rx, rx), -__fmul_rn(ry, ry));
-            z = jl_clamp(__fdiv_rn(__fmul_rn(-da, __fmul_rn(psf[7], psf[7])), __fmul_rn(4.0f, psf[6])),
-                         -600.f, 600.f);
-        }
-        th[2] = z;
-        th[3] = jl_maxf(total, 100.f);
-        th[4] = bg;
     }
+    warp_start<MODEL>(x, y, total, bg, mxx, myy, psf, th);
 }
 
 // Fit ROI `roi` of `a` with the calling warp; its shared memory is at `tab`.
@@ -252,7 +328,7 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
     const int lane = threadIdx.x & 31;
     const int ry = lane & (kRows - 1), rx = lane / kRows;
     const int B2 = box * box;
-    float *const spix = tab + 10 * box, *const svar = spix + B2;  // boxes beyond 32 only
+    float *const spix = tab + 10 * box, *const svar = spix + B2;  // (warp_floats)
     bool ok = true;
     long long base = 0;
     if (SCMOS) {
@@ -320,7 +396,13 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
     };
 
     float th[P];
-    warp_initialize<MODEL>(box, each, a.psf, th);
+    if constexpr (RMAX <= 4) {
+        each([&](int j, int i, float d) { spix[i + box * j] = d; });
+        __syncwarp();
+        warp_initialize_exact<MODEL>(box, each, spix, lane, a.psf, th);
+    } else {
+        warp_initialize<MODEL>(box, each, a.psf, th);
+    }
     float dmax = 0.f;  // Poisson: the largest pixel (NaN if any is), for uncapped()
     if (!SCMOS) {
         dmax = -INFINITY;
@@ -340,6 +422,7 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
     const int mine = min(unit, P - 1);
     const float lo = a.lower[mine], hi = a.upper[mine], most = a.max_step[mine];
     const int half = lane >> 4;  // 0: x axis, 1: y axis
+    const float nk = -__fdiv_rn(1.0f, a.sqrt2pi);
     float *const ytab = tab + 5 * box;
 
     for (int it = 0; it <= a.iterations; ++it) {
@@ -356,18 +439,23 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
                         half ? a.psf[3] : a.psf[2], half ? a.psf[5] : a.psf[4], a.psf[7], s,
                         w.ds, w.d2s);
         w.is = __fdiv_rn(1.0f, s);
-        w.cst = -N * __fdiv_rn(1.0f, a.sqrt2pi) * w.is;
+        w.cst = N * nk * w.is;
         __syncwarp();  // the previous pass has read the tables
-        for (int axis = 0; axis < 2; axis++) {
-            WarpAxis u;
-            u.c = __shfl_sync(0xffffffffu, w.c, 16 * axis);
-            u.is = __shfl_sync(0xffffffffu, w.is, 16 * axis);
-            u.cst = __shfl_sync(0xffffffffu, w.cst, 16 * axis);
-            u.ds = MODEL == 3 ? __shfl_sync(0xffffffffu, w.ds, 16 * axis) : 0.f;
-            u.d2s = MODEL == 3 ? __shfl_sync(0xffffffffu, w.d2s, 16 * axis) : 0.f;
-            for (int e0 = 0; e0 < box; e0 += 31) {
-                const int e = e0 + lane;
-                warp_entry<MODEL>(e, u, 32, lane < 31 && e < box, axis ? ytab : tab, box);
+        if (RMAX <= 4 && box <= 15) {  // both axes at once, at most 16 edges each
+            const int e = lane & 15;
+            warp_entry<MODEL>(e, w, 16, e < box, half ? ytab : tab, box);
+        } else {
+            for (int axis = 0; axis < 2; axis++) {
+                WarpAxis u;
+                u.c = __shfl_sync(0xffffffffu, w.c, 16 * axis);
+                u.is = __shfl_sync(0xffffffffu, w.is, 16 * axis);
+                u.cst = __shfl_sync(0xffffffffu, w.cst, 16 * axis);
+                u.ds = MODEL == 3 ? __shfl_sync(0xffffffffu, w.ds, 16 * axis) : 0.f;
+                u.d2s = MODEL == 3 ? __shfl_sync(0xffffffffu, w.d2s, 16 * axis) : 0.f;
+                for (int e0 = 0; e0 < box; e0 += 31) {
+                    const int e = e0 + lane;
+                    warp_entry<MODEL>(e, u, 32, lane < 31 && e < box, axis ? ytab : tab, box);
+                }
             }
         }
         __syncwarp();
@@ -563,20 +651,19 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
     }
 }
 
+// Fit the ROIs [roi0, roi0 + nroi) of `a`, one per warp of the block.
 template <int MODEL, bool SCMOS, int RMAX>
-__global__ void __launch_bounds__(128) fit_kernel_warp(const KernelArgs a, const int box)
+__device__ __forceinline__ void fit_block_warp(const KernelArgs &a, const int box,
+                                               const int64_t roi0, const int nroi, float *smem)
 {
     constexpr int P = ModelInfo<MODEL>::P;
-    __shared__ RoiResult<P> s_res[4];
-    extern __shared__ __align__(16) float smem[];
-    const int nw = blockDim.x >> 5, wid = threadIdx.x >> 5;
-    const int64_t roi0 = (int64_t)blockIdx.x * nw;
-    if (roi0 + wid < a.n)  // one decision per warp
+    __shared__ RoiResult<P> s_res[kWarpMaxRois];
+    const int wid = threadIdx.x >> 5;
+    if (wid < nroi)  // one decision per warp
         fit_roi_warp<MODEL, SCMOS, RMAX>(a, box, roi0 + wid,
                                          smem + (size_t)wid * warp_floats(box, SCMOS), s_res[wid]);
     __syncthreads();
-    const int64_t out = roi0 + threadIdx.x;
-    if (threadIdx.x < nw && out < a.n) {
+    if (threadIdx.x < nroi) {
         const RoiResult<P> &res = s_res[threadIdx.x];
         double Fm[P][P];
         float th[P];
@@ -587,21 +674,46 @@ __global__ void __launch_bounds__(128) fit_kernel_warp(const KernelArgs a, const
 #pragma unroll
             for (int l = k; l < P; l++, q++) Fm[k][l] = Fm[l][k] = res.F[q];
         }
-        write_result<P>(a, out, res.ok, th, Fm, res.llr);
+        write_result<P>(a, roi0 + threadIdx.x, res.ok, th, Fm, res.llr);
     }
 }
 
-using WarpKernel = void (*)(const KernelArgs, const int);
+// TABLE as for fit_kernel_r1, with tiles of one ROI per warp (boxes up to 16).
+template <int MODEL, bool SCMOS, int RMAX, bool TABLE>
+__global__ void __launch_bounds__(32 * kWarpMaxRois)
+    fit_kernel_warp(const KernelArgs a, const TileTable t, const int box)
+{
+    extern __shared__ __align__(16) float smem[];
+    const int nw = blockDim.x >> 5;
+    if (!TABLE) {
+        const int64_t roi0 = (int64_t)blockIdx.x * nw, left = a.n - roi0;
+        fit_block_warp<MODEL, SCMOS, RMAX>(a, box, roi0, left < nw ? (int)left : nw, smem);
+    } else {
+        TableSlot *ts = table_slot(smem, sizeof(float) * (size_t)warp_floats(box, SCMOS) * nw);
+        table_slot_init(ts);
+        int64_t roi0;
+        int nroi;
+        for (int k = 0; table_next(t, nw, ts, k, roi0, nroi); k++) {
+            fit_block_warp<MODEL, SCMOS, RMAX>(ts->a, box, roi0, nroi, smem);
+            __syncthreads();  // the tile's shared memory and slot are free again
+        }
+    }
+}
 
-template <int MODEL, bool SCMOS> WarpKernel warp_kernel(int box)
+using WarpKernel = void (*)(const KernelArgs, const TileTable, const int);
+
+template <int MODEL, bool SCMOS> WarpKernel warp_kernel(int box, bool table)
 {
     switch (rows_per_lane(box)) {
-        case 5: return fit_kernel_warp<MODEL, SCMOS, 5>;
-        case 6: return fit_kernel_warp<MODEL, SCMOS, 6>;
-        case 7: return fit_kernel_warp<MODEL, SCMOS, 7>;
-        case 8: return fit_kernel_warp<MODEL, SCMOS, 8>;
-        case 12: return fit_kernel_warp<MODEL, SCMOS, 12>;
-        case 16: return fit_kernel_warp<MODEL, SCMOS, 16>;
+        case 2: return table ? fit_kernel_warp<MODEL, SCMOS, 2, true> : fit_kernel_warp<MODEL, SCMOS, 2, false>;
+        case 3: return table ? fit_kernel_warp<MODEL, SCMOS, 3, true> : fit_kernel_warp<MODEL, SCMOS, 3, false>;
+        case 4: return table ? fit_kernel_warp<MODEL, SCMOS, 4, true> : fit_kernel_warp<MODEL, SCMOS, 4, false>;
+        case 5: return table ? nullptr : fit_kernel_warp<MODEL, SCMOS, 5, false>;
+        case 6: return table ? nullptr : fit_kernel_warp<MODEL, SCMOS, 6, false>;
+        case 7: return table ? nullptr : fit_kernel_warp<MODEL, SCMOS, 7, false>;
+        case 8: return table ? nullptr : fit_kernel_warp<MODEL, SCMOS, 8, false>;
+        case 12: return table ? nullptr : fit_kernel_warp<MODEL, SCMOS, 12, false>;
+        case 16: return table ? nullptr : fit_kernel_warp<MODEL, SCMOS, 16, false>;
         default: return nullptr;
     }
 }
@@ -609,24 +721,42 @@ template <int MODEL, bool SCMOS> WarpKernel warp_kernel(int box)
 }  // namespace
 
 template <int MODEL, bool SCMOS>
-cudaError_t launch_warp_family(int box, const KernelArgs &a, int rois_per_block, cudaStream_t s)
+cudaError_t launch_warp_family(int box, const KernelArgs &a, const TileTable &t,
+                               int rois_per_block, int64_t grid, cudaStream_t s)
 {
-    WarpKernel k = warp_kernel<MODEL, SCMOS>(box);
-    if (!k || rois_per_block < 1 || rois_per_block > 4) return cudaErrorInvalidValue;
-    const size_t smem = sizeof(float) * (size_t)warp_floats(box, SCMOS) * rois_per_block;
-    if (smem > 48 * 1024) {
+    const bool table = t.header != nullptr;
+    if (box < 3 || box > kLargeMaxBox || a.tpr != 32) return cudaErrorInvalidValue;
+    WarpKernel k = warp_kernel<MODEL, SCMOS>(box, table);
+    if (!k || rois_per_block < 1 || rois_per_block > kWarpMaxRois)
+        return cudaErrorInvalidValue;
+    size_t smem = sizeof(float) * (size_t)warp_floats(box, SCMOS) * rois_per_block;
+    if (table) smem = table_smem_bytes(smem);
+    if (smem > 48 * 1024 - 4096) {  // (the kernel's static shared memory counts as well)
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
         if (e != cudaSuccess) return e;
     }
-    const int64_t blocks = (a.n + rois_per_block - 1) / rois_per_block;
+    const int64_t blocks = table ? grid : (a.n + rois_per_block - 1) / rois_per_block;
     if (blocks <= 0) return cudaSuccess;
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    k<<<(unsigned)blocks, 32 * rois_per_block, smem, s>>>(a, box);
+    k<<<(unsigned)blocks, 32 * rois_per_block, smem, s>>>(a, t, box);
     return cudaGetLastError();
 }
 
-template cudaError_t launch_warp_family<GMLE_MODEL, (GMLE_SCMOS != 0)>(int, const KernelArgs &, int,
-                                                                      cudaStream_t);
+template <int MODEL, bool SCMOS> int warp_table_blocks(int box, int rois_per_block)
+{
+    WarpKernel k = warp_kernel<MODEL, SCMOS>(box, true);
+    if (!k) return 0;
+    int nb = 0;
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &nb, k, 32 * rois_per_block,
+        table_smem_bytes(sizeof(float) * (size_t)warp_floats(box, SCMOS) * rois_per_block));
+    return e == cudaSuccess ? nb : -(int)e;
+}
+
+template cudaError_t launch_warp_family<GMLE_MODEL, (GMLE_SCMOS != 0)>(int, const KernelArgs &,
+                                                                      const TileTable &, int,
+                                                                      int64_t, cudaStream_t);
+template int warp_table_blocks<GMLE_MODEL, (GMLE_SCMOS != 0)>(int, int);
 
 }  // namespace gmle

@@ -12,7 +12,6 @@
 
 #include "../../include/gaussmle_gb300.h"
 #include "gmle_launch.cuh"
-#include "gmle_warp.h"
 
 namespace gmle_rt {
 
@@ -46,6 +45,9 @@ struct Slot {
 // Launch kinds of a mixed batch: one table launch per (camera family, PSF
 // model, box size) present.
 constexpr int kKinds = 2 * 4 * gmle::kNumBoxes;
+// A serving step may have two launches of a kind, of small and of large requests:
+// table k of a kind's small (or only) requests, k + kKinds of its large ones.
+constexpr int kTables = 2 * kKinds;
 inline int kind_of(const gmle_fit_desc &d)
 {
     return ((d.camera != GMLE_CAMERA_POISSON) * 4 + d.model) * gmle::kNumBoxes +
@@ -77,7 +79,7 @@ struct TableBufs {
 // context's synchronous path, or one slot of the serving loop).
 constexpr int kForks = 4;
 struct MixedSet {
-    TableBufs tables[kKinds];
+    TableBufs tables[kTables];
     // The kernels read the tables from pinned host memory (no copy).  The
     // serving loop does so: a table copy would queue on the copy engine
     // behind the inputs of every admitted request.
@@ -95,7 +97,7 @@ struct MixedSet {
 
 // One table launch of a plan.
 struct TableLaunch {
-    int kind = -1, model = 0, box = 0;
+    int table = -1, model = 0, box = 0;
     bool scmos = false;
     bool persistent = true;  // false: one block per tile (no tile counter)
     gmle::LaunchShape shape{};
@@ -147,16 +149,20 @@ int nparams(int model);
 
 gmle_status init_mixed_set(gmle_ctx *ctx, MixedSet &m);
 void free_mixed_set(MixedSet &m);
-// How a table launch picks its shape: from the context's tuning for the
-// kind, else the size-based default for a submission of `shape_rois` ROIs (0:
-// this one's), with `line` ROIs per SM from which one thread fits a ROI
-// (default_tuning).  Persistent grids are full (SMs x resident blocks)
-// when `full_grid`, else no larger than the tiles.
-constexpr int kPlainLine = 80, kServingLine = 80, kSubmissionLine = 200;
+// ROIs per SM up to which a warp fits a ROI (alone, and of a submission whose
+// launches share the GPU), and from which one thread does (default_tuning).
+constexpr int kWarpLine = 16, kWarpTogether = 20, kPlainLine = 80, kSubmissionLine = 200;
+// How a table launch picks its shape: from the context's tuning for the kind,
+// else the size-based default for a submission of `shape_rois` ROIs (0: this
+// one's); with request_rois > 0 by each group's own size instead, so that
+// a request's results do not depend on what it is submitted with: one thread
+// per ROI up to boxes of large_box pixels and from that many ROIs, four lanes
+// otherwise.  Persistent grids are full
+// (SMs x resident blocks) when `full_grid`, else no larger than the tiles.
 struct PlanOptions {
     bool allow_plain = true;
-    int64_t shape_rois = 0;
-    int line = kSubmissionLine;
+    int64_t shape_rois = 0, request_rois = 0;
+    int large_box = 0;
     // persistent table launches (a grid of resident blocks that take tiles from
     // a counter; full_grid: sized for the GPU whatever the tiles) or one block
     // per tile
@@ -183,10 +189,8 @@ gmle_status enqueue_table_launch(gmle_ctx *ctx, MixedSet &m, const TableLaunch &
 // m.fork when there are several, joined back into s.
 gmle_status enqueue_plan(gmle_ctx *ctx, MixedSet &m, const MixedPlan &plan, cudaStream_t s);
 gmle_status validate_groups(gmle_ctx *ctx, const gmle_group *groups, int32_t ngroups);
-Tuning pick_tuning(gmle_ctx *ctx, const gmle_fit_desc *d, int64_t n, int64_t together = 0,
-                   int line = kPlainLine);
-Tuning default_tuning(int num_sms, int model, int box, bool scmos, int64_t n, int64_t together = 0,
-                      int line = kPlainLine);
+Tuning pick_tuning(gmle_ctx *ctx, const gmle_fit_desc *d, int64_t n, int64_t together = 0);
+Tuning default_tuning(int num_sms, int box, bool scmos, int64_t n, int64_t together = 0);
 gmle::KernelArgs make_args(gmle_ctx *ctx, const gmle_fit_desc *d, const float *data,
                            const int32_t *xc, const int32_t *yc, int64_t n, float *params,
                            float *crlb, float *llr, uint8_t *flags, int tpr);

@@ -14,6 +14,7 @@
 #include <algorithm>
 
 #include "gmle_fit_kernel.cuh"
+#include "gmle_warp.h"
 
 namespace gmle {
 
@@ -50,8 +51,9 @@ struct LaunchShape {
     bool lm = false;
 };
 
-// Lanes per ROI with a compiled kernel: 1 (fit_kernel_r1) for every box; 4
-// (fit_kernel) for every box; 2 and 8 for the odd boxes 5..15.
+// Lanes per ROI with a specialised kernel: 1 (fit_kernel_r1) for every box; 4
+// (fit_kernel) for every box; 2 and 8 for the odd boxes 5..15.  (A whole warp,
+// 32, is gmle_fit_warp.cu's.)
 inline bool tpr_supported(int tpr, int box)
 {
     return tpr == 1 || tpr == 4 || ((tpr == 2 || tpr == 8) && main_box(box));
@@ -69,6 +71,8 @@ int table_blocks_part(int box, int tpr, int rois_per_block);
 inline cudaError_t launch_fit(int model, int box, bool scmos, const KernelArgs &a,
                               const TileTable &t, const LaunchShape &shape, cudaStream_t s)
 {
+    if (shape.tpr == 32 && !shape.lm)
+        return launch_fit_warp(model, box, scmos, a, t, shape.rois_per_block, shape.grid, s);
     if (!box_supported(box) || !tpr_supported(shape.tpr, box)) return cudaErrorInvalidValue;
     const int part = part_of(box, shape.tpr);
 #define GMLE_CASE(M)                                                                       \
@@ -93,6 +97,8 @@ inline cudaError_t launch_fit(int model, int box, bool scmos, const KernelArgs &
 // the current device.
 inline int table_blocks_per_sm(int model, int box, bool scmos, int tpr, int rois_per_block)
 {
+    if (tpr == 32 && box_supported(box))
+        return warp_table_blocks_per_sm(model, box, scmos, rois_per_block);
     if (!box_supported(box) || !tpr_supported(tpr, box)) return -(int)cudaErrorInvalidValue;
     const int part = part_of(box, tpr);
 #define GMLE_CASE(M)                                                                       \

@@ -219,18 +219,13 @@ extern "C" gmle_status gmle_fit_mixed_device_noalloc(const gmle_group *groups, i
     gmle::LaunchShape shape[kKinds] = {};
     for (int kind = 0; kind < kKinds; kind++) {
         int cnt = 0;
-        int64_t rois = 0;
         for (int k = 0; k < ngroups; k++)
-            if (groups[k].n > 0 && gmle_rt::kind_of(groups[k].desc) == kind) {
-                g_order[cnt++] = k;
-                rois += groups[k].n;
-            }
+            if (groups[k].n > 0 && gmle_rt::kind_of(groups[k].desc) == kind) g_order[cnt++] = k;
         first[kind] = used;
         if (cnt == 0) continue;
         const gmle_fit_desc &d0 = groups[g_order[0]].desc;
         const bool scmos = d0.camera != GMLE_CAMERA_POISSON;
-        const gmle_rt::Tuning t = gmle_rt::default_tuning(S.num_sms, d0.model, d0.box, scmos, rois,
-                                                             together, gmle_rt::kSubmissionLine);
+        const gmle_rt::Tuning t = gmle_rt::default_tuning(S.num_sms, d0.box, scmos, together, together);
         int64_t tiles = 0;
         for (int q = 0; q < cnt; q++) {
             const gmle_group &G = groups[g_order[q]];

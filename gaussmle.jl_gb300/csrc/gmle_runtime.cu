@@ -94,11 +94,16 @@ namespace gmle_rt {
 // 300 000: 1208 / 610 and 2295 / 1112.  The line is drawn at 80 ROIs per SM.
 //
 // `together` > 0: the launch is one of several, of `together` ROIs in all, that
-// share the SMs.  A submission that waits for its slowest launch (`line` 200 ROIs
-// per SM) gains from short chains for longer than serving steps that overlap
-// (80).  Measured on the five kinds of the sCMOS mixed batch (us, 4 lanes / one
-// thread): 12 000 ROIs 187 / 295, 25 000 246 / 294, 50 000 421 / 313; served
-// requests of 12 000 ROIs 387 / 394, 25 000 461 / 394, 100 000 968 / 774.
+// share the SMs and are waited for together: the slowest launch's chain counts
+// for longer.  Measured on the five kinds of the sCMOS mixed batch (us, 4 lanes /
+// one thread): 12 000 ROIs 187 / 295, 25 000 246 / 294, 50 000 421 / 313.  That
+// line is drawn at 200 ROIs per SM.
+//
+// Up to 16 ROIs per SM (20 in a submission of several launches) a warp fits a
+// ROI: a pass is then a few hundred cycles instead of over a thousand, and all
+// warps are resident at once.  Measured (us, 4 lanes / 8 lanes / a warp): 200 ROIs
+// XYNB 11x11 45 / 43 / 23, astigmatic 15x15 99 / 72 / 37; 2 400 ROIs 45 / 43 / 31 and
+// 100 / 72 / 54; 3 000 ROIs, in two waves of warps, astigmatic 101 / 90 / 84.
 //
 // ROIs per block of the one-thread kernel: with sCMOS data 128, whose four warps
 // use their tensor-memory columns fully; Poisson data the block that lets
@@ -107,17 +112,20 @@ namespace gmle_rt {
 // which fit).  Below 256 ROIs per SM smaller blocks spread over the SMs evenly
 // (20 000 XYNB 11x11 ROIs: 98 us in blocks of 32; 40 000 11x11 sCMOS: 131 us in
 // blocks of 96, 137 us of 128).
-Tuning default_tuning(int num_sms, int model, int box, bool scmos, int64_t n, int64_t together,
-                      int line)
+Tuning default_tuning(int num_sms, int box, bool scmos, int64_t n, int64_t together)
 {
-    if ((together > 0 ? together : n) < (int64_t)line * num_sms) return {4, 32};
+    const int64_t all = together > 0 ? together : n;
+    const int line = together > 0 ? kSubmissionLine : kPlainLine;
+    if (all < (int64_t)(together > 0 ? kWarpTogether : kWarpLine) * num_sms)
+        return {32, gmle::warp_rois_per_block(num_sms, box, scmos, all)};
+    if (all < (int64_t)line * num_sms) return {4, 32};
     const bool spread = together == 0 && n < (int64_t)256 * num_sms;
     if (scmos) return {1, spread ? 96 : 128};
     if (spread) return {1, 32};
     int best = 64, most = 0;
     for (int rpb : {64, 128, 32}) {
         // a block takes 1 KiB beside its own shared memory of the SM's 228 KiB
-        const size_t block = gmle::smem_bytes(model, box, scmos, 1, rpb) + 1024;
+        const size_t block = gmle::smem_bytes(0, box, scmos, 1, rpb) + 1024;
         const int rois = rpb * (int)(228 * 1024 / block);
         if (rois > most) { most = rois; best = rpb; }
     }
@@ -128,14 +136,13 @@ Tuning default_tuning(int num_sms, int model, int box, bool scmos, int64_t n, in
 
 namespace gmle_rt {
 
-Tuning pick_tuning(gmle_ctx *ctx, const gmle_fit_desc *d, int64_t n, int64_t together, int line)
+Tuning pick_tuning(gmle_ctx *ctx, const gmle_fit_desc *d, int64_t n, int64_t together)
 {
     const bool scmos = d->camera != GMLE_CAMERA_POISSON;
-    if (gmle::large_box(d->box)) return {32, gmle::warp_rois_per_block(d->box, scmos)};
+    if (gmle::large_box(d->box)) return {32, gmle::warp_rois_per_block(ctx->num_sms, d->box, scmos, n)};
     auto it = ctx->tuning.find({d->model, d->box, (int)scmos});
     Tuning t = it != ctx->tuning.end() ? it->second
-                                       : default_tuning(ctx->num_sms, d->model, d->box, scmos, n,
-                                                        together, line);
+                                       : default_tuning(ctx->num_sms, d->box, scmos, n, together);
     if (d->method == GMLE_METHOD_FISHER_LM && t.tpr != 1) {
         // the full-Hessian method runs one thread per ROI; 128-thread blocks
         // use the tensor memory of sCMOS variance tiles fully
@@ -186,7 +193,6 @@ cudaError_t launch(gmle_ctx *ctx, const gmle_fit_desc *d, const KernelArgs &a, i
 {
     const bool scmos = d->camera != GMLE_CAMERA_POISSON;
     ctx->launches++;
-    if (a.tpr == 32) return gmle::launch_fit_warp(d->model, d->box, scmos, a, rpb, s);
     gmle::LaunchShape shape{a.tpr, rpb, 0};
     shape.lm = d->method == GMLE_METHOD_FISHER_LM;
     return gmle::launch_fit(d->model, d->box, scmos, a, gmle::TileTable{}, shape, s);
@@ -519,7 +525,7 @@ gmle_status gmle_get_tuning(gmle_ctx *ctx, int32_t model, int32_t box, int32_t c
     const bool scmos = camera != GMLE_CAMERA_POISSON;
     auto it = ctx->tuning.find({model, box, (int)scmos});
     Tuning t = it != ctx->tuning.end() ? it->second
-                                       : default_tuning(ctx->num_sms, model, box, scmos, 1ll << 40);
+                                       : default_tuning(ctx->num_sms, box, scmos, 1ll << 40);
     *threads_per_roi = t.tpr;
     *rois_per_block = t.rois_per_block;
     return GMLE_OK;
@@ -761,8 +767,8 @@ gmle_status plan_mixed(gmle_ctx *ctx, const gmle_group *groups, int32_t ngroups,
     if (st != GMLE_OK) return st;
     plan = MixedPlan();
     m.pool_used = 0;
-    std::vector<int> by_kind[kKinds];
-    int64_t rois[kKinds] = {}, together = 0;
+    std::vector<int> by_table[kTables];
+    int64_t together = 0;
     for (int k = 0; k < ngroups; k++) {
         const gmle_group &G = groups[k];
         if (G.n <= 0) continue;
@@ -771,25 +777,32 @@ gmle_status plan_mixed(gmle_ctx *ctx, const gmle_group *groups, int32_t ngroups,
             plan.plain.push_back(G);
             continue;
         }
-        const int kind = kind_of(G.desc);
-        by_kind[kind].push_back(k);
-        rois[kind] += G.n;
+        // (a tuned shape is every request's)
+        const bool large = opt.request_rois > 0 &&
+                           (G.desc.box <= opt.large_box || G.n >= opt.request_rois) &&
+                           !ctx->tuning.count({G.desc.model, G.desc.box,
+                                               (int)(G.desc.camera != GMLE_CAMERA_POISSON)});
+        by_table[kind_of(G.desc) + (large ? kKinds : 0)].push_back(k);
     }
-    for (int kind = 0; kind < kKinds; kind++) {
-        if (by_kind[kind].empty()) continue;
-        const gmle_fit_desc &d0 = groups[by_kind[kind][0]].desc;
+    for (int table = 0; table < kTables; table++) {
+        const std::vector<int> &members = by_table[table];
+        if (members.empty()) continue;
+        const gmle_fit_desc &d0 = groups[members[0]].desc;
         TableLaunch L;
-        L.kind = kind;
+        L.table = table;
         L.model = d0.model;
         L.box = d0.box;
         L.scmos = d0.camera != GMLE_CAMERA_POISSON;
-        const Tuning t = pick_tuning(ctx, &d0, rois[kind],
-                                     opt.shape_rois > 0 ? opt.shape_rois : together, opt.line);
+        const int64_t all =
+            opt.request_rois > 0
+                ? (int64_t)(table >= kKinds ? kSubmissionLine : kWarpTogether) * ctx->num_sms
+            : opt.shape_rois > 0 ? opt.shape_rois : together;
+        const Tuning t = pick_tuning(ctx, &d0, all, all);
         const int rpb = t.rois_per_block;
         int64_t tiles = 0;
-        for (int k : by_kind[kind]) tiles += (groups[k].n + rpb - 1) / rpb;
-        TableBufs &b = m.tables[kind];
-        const int64_t ng = (int64_t)by_kind[kind].size();
+        for (int k : members) tiles += (groups[k].n + rpb - 1) / rpb;
+        TableBufs &b = m.tables[table];
+        const int64_t ng = (int64_t)members.size();
         const size_t need = (kTableHeader + sizeof(KernelArgs) * (size_t)ng + sizeof(int64_t) * (size_t)tiles +
                              255) & ~size_t(255);
         if (m.pool && m.zero_copy && !opt.persistent && m.pool_used + need <= m.pool_bytes) {
@@ -811,15 +824,15 @@ gmle_status plan_mixed(gmle_ctx *ctx, const gmle_group *groups, int32_t ngroups,
         KernelArgs *args = reinterpret_cast<KernelArgs *>(b.h_base + kTableHeader);
         int64_t *map = reinterpret_cast<int64_t *>(b.h_base + b.tiles_off());
         int64_t tile = 0;
-        for (size_t q = 0; q < by_kind[kind].size(); q++) {
-            const gmle_group &G = groups[by_kind[kind][q]];
+        for (size_t q = 0; q < members.size(); q++) {
+            const gmle_group &G = groups[members[q]];
             args[q] = make_args(ctx, &G.desc, G.data, G.x_corners, G.y_corners, G.n, G.params,
                                 G.crlb, G.llr, G.flags, t.tpr);
             const int64_t nt = (G.n + rpb - 1) / rpb;
             for (int64_t j = 0; j < nt; j++) map[tile + j] = ((int64_t)q << 32) | j;
             tile += nt;
         }
-        hdr[0] = (int64_t)by_kind[kind].size();
+        hdr[0] = (int64_t)members.size();
         hdr[1] = tiles;
         const int bps = gmle::table_blocks_per_sm(L.model, L.box, L.scmos, t.tpr, rpb);
         if (bps <= 0)
@@ -843,7 +856,7 @@ gmle_status upload_plan(gmle_ctx *ctx, MixedSet &m, const MixedPlan &plan, cudaS
 {
     if (m.zero_copy) return GMLE_OK;
     for (const TableLaunch &L : plan.launches) {
-        TableBufs &b = m.tables[L.kind];
+        TableBufs &b = m.tables[L.table];
         // the device table is rewritten after the last launch that read it
         CK(cudaStreamWaitEvent(s, b.used, 0), "cudaStreamWaitEvent");
         CK(cudaMemcpyAsync(b.d_base, b.h_base, kTableHeader + sizeof(KernelArgs) * L.groups,
@@ -857,7 +870,7 @@ gmle_status upload_plan(gmle_ctx *ctx, MixedSet &m, const MixedPlan &plan, cudaS
 
 gmle_status enqueue_table_launch(gmle_ctx *ctx, MixedSet &m, const TableLaunch &L, cudaStream_t q)
 {
-    TableBufs &b = m.tables[L.kind];
+    TableBufs &b = m.tables[L.table];
     const char *base = m.zero_copy ? b.h_base : b.d_base;
     gmle::TileTable t;
     t.header = reinterpret_cast<const int64_t *>(base);

@@ -51,6 +51,15 @@ constexpr int kMaxSlots = 8;
 // a launch could then wait behind an unrelated one.
 constexpr int kRunStreams = 6;
 constexpr int kServerTableCap = 4096;  // groups (requests) per step and kind
+// Requests of this many ROIs, and of boxes up to 10 pixels, are fitted with one
+// thread per ROI, the others with four lanes: by the request's own size, so that
+// its results do not depend on the step it runs in.  One thread takes half the
+// work per ROI and, for the large boxes, a third longer (astigmatic 15x15: 150 us
+// against 103): 100 000 sCMOS ROIs in 10 requests 786 us with four lanes for all
+// boxes above 10, 658 us so; in 40 requests 894 and 861; with the line at 1 000
+// ROIs 777, but 18 000 ROIs in 17 requests went from 386 to 485.
+constexpr int64_t kLargeRequest = 4000;
+constexpr int kLargeRequestBox = 10;
 constexpr size_t kLatencyRecord = 1 << 20;  // latencies kept for the percentiles
 
 enum ReqState { PENDING, STAGED, RUNNING, DRAINING, DONE, FAILED };
@@ -155,9 +164,9 @@ struct Server {
     cudaStream_t s_run[kRunStreams] = {};
     cudaStream_t s_capture = nullptr;  // graph capture only: never runs work
     int next_run = 0;
-    // per slot and kind: the event after that kind's launch (scheduler thread
-    // only, created on first use; a slot's step has at most one launch per kind)
-    cudaEvent_t launch_done[kMaxSlots][kKinds] = {};
+    // per slot and table: the event after that table's launch (scheduler thread
+    // only, created on first use; a slot's step has at most one launch per table)
+    cudaEvent_t launch_done[kMaxSlots][kTables] = {};
     bool slot_busy[kMaxSlots] = {};
     MixedSet sets[kMaxSlots];
     // per slot and kind: the captured counter reset + table launch, and the
@@ -166,7 +175,7 @@ struct Server {
         std::vector<int64_t> key;
         cudaGraphExec_t exec = nullptr;
     };
-    KindGraph graphs[kMaxSlots][kKinds];
+    KindGraph graphs[kMaxSlots][kTables];
     // statistics
     int64_t submitted = 0, completed = 0, rejected = 0, failed = 0, rois_done = 0, steps = 0;
     std::vector<float> lat_ms;
@@ -352,7 +361,8 @@ struct Server {
     }
 
     // One step: the tables of every kind in the slot's pinned buffers (read
-    // in place by the kernels), then one launch per kind present, spread over
+    // in place by the kernels), then one launch per kind present (two when it has
+    // both small and large requests), spread over
     // the run streams, each followed by an event in `done`.  Direct launches
     // have one block per tile.  With graphs, each launch is a replay of the
     // slot's graph of a persistent launch for that kind (captured on first
@@ -371,8 +381,9 @@ struct Server {
         std::lock_guard<std::mutex> lk(ctx->mu);
         PlanOptions opt;
         opt.allow_plain = false;
-        opt.shape_rois = cfg.use_graphs ? cfg.max_step_rois : 0;
-        opt.line = kServingLine;
+        opt.shape_rois = cfg.max_step_rois;
+        opt.request_rois = cfg.use_graphs ? 0 : kLargeRequest;
+        opt.large_box = kLargeRequestBox;
         // a graph replays a fixed grid: persistent launches; direct launches
         // take one block per tile
         opt.persistent = cfg.use_graphs != 0;
@@ -393,11 +404,11 @@ struct Server {
                 st = enqueue_table_launch(ctx, m, L, q);
                 if (st != GMLE_OK) return st;
             } else {
-                const TableBufs &b = m.tables[L.kind];
+                const TableBufs &b = m.tables[L.table];
                 const std::vector<int64_t> key = {L.shape.tpr, L.shape.rois_per_block,
                                                   L.shape.grid, (int64_t)(uintptr_t)b.h_base,
                                                   b.cap_groups};
-                KindGraph &kg = graphs[slot][L.kind];
+                KindGraph &kg = graphs[slot][L.table];
                 if (!kg.exec || kg.key != key) {
                     if (kg.exec) cudaGraphExecDestroy(kg.exec);
                     kg.exec = nullptr;
@@ -420,7 +431,7 @@ struct Server {
                 GMLE_CK(cudaGraphLaunch(kg.exec, q), "cudaGraphLaunch");
                 ctx->launches++;
             }
-            cudaEvent_t &ev = launch_done[slot][L.kind];
+            cudaEvent_t &ev = launch_done[slot][L.table];
             if (!ev)
                 GMLE_CK(cudaEventCreateWithFlags(&ev, tracing() ? cudaEventDefault
                                                                 : cudaEventDisableTiming),
@@ -677,8 +688,8 @@ gmle_status gmle_server_start(gmle_ctx *ctx, const gmle_server_config *config)
     // that no step allocates: a first allocation would synchronise the device
     // mid-stream.  Graph replays keep a table per kind at a fixed address.
     const size_t pool_bytes =
-        ((kTableHeader + 256) * kKinds + sizeof(gmle::KernelArgs) * (size_t)kServerTableCap +
-         sizeof(int64_t) * (size_t)(S->cfg.max_step_rois / 16 + kServerTableCap + kKinds) + 4095) &
+        ((kTableHeader + 256) * kTables + sizeof(gmle::KernelArgs) * (size_t)kServerTableCap +
+         sizeof(int64_t) * (size_t)(S->cfg.max_step_rois / 16 + kServerTableCap + kTables) + 4095) &
         ~size_t(4095);
     for (int k = 0; ok && k < S->cfg.max_inflight_steps; k++) {
         S->sets[k].zero_copy = true;

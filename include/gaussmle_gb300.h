@@ -346,8 +346,9 @@ gmle_status gmle_fit_mixed_device_noalloc(const gmle_group *groups, int32_t ngro
  * per batch, src/interface.jl:220-262).  A scheduler thread owned by the
  * context admits submitted requests into a device arena (admission by HBM
  * budget, FIFO), copies their ROIs in, and continuously batches every request
- * whose data has arrived into the next step: one table launch per (camera
- * family, model, box) present, with one block per tile of 32..128 ROIs.  Up
+ * whose data has arrived into the next step: one or two table launches
+ * per (camera family, model, box) present, with one block per tile of 32..128
+ * ROIs.  Up
  * to max_inflight_steps steps run concurrently, and their blocks interleave
  * on the SMs, so requests that arrive while others are on the GPU start as
  * soon as SMs and memory free up.  Results land in the caller's host
