@@ -152,140 +152,128 @@ __device__ __forceinline__ float gauss_edge(float t)
 {
     return ex2_approx(__fmul_rn(t, t) * -0.72134752044448170368f);
 }
-// erf(x), given e = exp(-x^2) (the caller's gauss_edge at the same edge).
-// Hastings' form (Abramowitz & Stegun 7.1.26): erf(|x|) = 1 - e t P(t) with
-// t = 1 / (1 + p |x|), here with P of degree 5 refitted by a least-squares
-// (Lawson) minimax fit of exp(-x^2) erfcx(x) on [0, 6]: p = 0.39, 8.3e-9 largest
-// error in exact arithmetic, below 4e-7 absolute evaluated in FP32 (most of it
-// near x = 0, from 1 - e t P(t)); erf(-x) = -erf(x).  Checked against the
-// library's erff by tests/test_math_gpu.py.
-__device__ __forceinline__ float erf_from_gauss(float x, float e)
+// erf(t / sqrt 2) / 2, given f = exp(-t^2 / 2) (the caller's gauss_edge at the
+// same edge).  Hastings' form (Abramowitz & Stegun 7.1.26): erf(x) = 1 - e r P(r)
+// for x >= 0, e = exp(-x^2), r = 1 / (1 + p x), here with P of degree 5 refitted
+// by a least-squares (Lawson) minimax fit of exp(-x^2) erfcx(x) on [0, 6]: p =
+// 0.39, 8.3e-9 largest error in exact arithmetic, below 4.5e-7 absolute (of erf)
+// evaluated in FP32 (most of it near x = 0, from 1 - e r P(r)); erf(-x) =
+// -erf(x).  The factor 1/2 is in P's coefficients, 1/sqrt 2 in p.  Checked against
+// the library's erff by tests/test_math_gpu.py.
+__device__ __forceinline__ float half_erf(float t, float f)
 {
-    const float t = rcp_approx(fmaf(0.39f, fabsf(x), 1.0f));
-    float p = -0.22753699123859406f;
-    p = fmaf(p, t, 0.8866637945175171f);
-    p = fmaf(p, t, -0.6353994011878967f);
-    p = fmaf(p, t, 0.6495586633682251f);
-    p = fmaf(p, t, 0.09138870239257812f);
-    p = fmaf(p, t, 0.2353251725435257f);
-    return copysignf(fmaf(-e, t * p, 1.0f), x);
+    const float r = rcp_approx(fmaf(0.27577164466275354f, fabsf(t), 1.0f));
+    float p = 0.5f * -0.22753699123859406f;
+    p = fmaf(p, r, 0.5f * 0.8866637945175171f);
+    p = fmaf(p, r, 0.5f * -0.6353994011878967f);
+    p = fmaf(p, r, 0.5f * 0.6495586633682251f);
+    p = fmaf(p, r, 0.5f * 0.09138870239257812f);
+    p = fmaf(p, r, 0.5f * 0.2353251725435257f);
+    return copysignf(fmaf(-f, r * p, 0.5f), t);
 }
 
 // ---- per-axis coefficients (hoisted out of the pixel loops) ----------------
 
 struct Axis {
-    float c;     // centre (x or y, ROI pixels)
-    float s;     // sigma (pixels)
-    float inv_s; // 1 / s
-    float sq;    // sqrt(0.5 / s^2): integral_gaussian_1d, baselibrary.jl:8-14
-    float cst;   // (-N / sqrt(2pi)) / s: derivative_integral_gaussian_1d, baselibrary.jl:21-33
-    float cst2;  // cst / s^2
-    float s1c;   // ((-N / sqrt(2pi)) / s) / s: baselibrary.jl:40-52 (dudt)
-    float s2c;   // (N / sqrt(2pi)) / s^5            (d2udt2 second term)
-    float m2s;   // -2 / s                             (d2udt2 first factor)
+    float c;           // centre (x or y, ROI pixels)
+    float inv_s;       // 1 / sigma (pixels)
+    float cst;         // -N / (sqrt(2 pi) s): derivative_integral_gaussian_1d, baselibrary.jl:21-33
+    float cst2;        // cst / s^2
+    // derivatives by the width's parameter (s itself, or z): baselibrary.jl:40-52
+    // and the chain rule of src/psf_derivatives.jl:118-163, as coefficients of the
+    // differences of u f and u^3 f between a pixel's edges
+    float kz, kq, kq3;
 };
 
-__device__ __forceinline__ Axis make_axis(float c, float s, float N, float sqrt2pi, bool sig)
+// cst = -N / sqrt(2 pi) / s; ds, d2s: the astigmatic width's derivatives by z.
+// One division per axis (1/s); the other factors are products of it, each within
+// a few ulp of the reference's chained divisions.
+template <int MODEL>
+__device__ __forceinline__ Axis make_axis(float c, float inv_s, float cst, float ds, float d2s)
 {
-    // One division per axis; the remaining factors are products of 1/s, each
-    // within a few ulp of the reference's chained divisions.
     Axis a;
     a.c = c;
-    a.s = s;
-    const float is = __fdiv_rn(1.0f, s);
-    a.inv_s = is;
-    const float is2 = is * is;
-    a.sq = 0.70710678118654752f * is;                 // sqrt(1/2 / s^2), s > 0
-    const float nk = -N * __fdiv_rn(1.0f, sqrt2pi);   // -N / sqrt(2 pi)
-    a.cst = nk * is;
-    a.cst2 = a.cst * is2;
-    if (sig) {
-        a.s1c = a.cst * is;
-        a.s2c = -nk * (is2 * is2 * is);
-        a.m2s = -2.0f * is;
-    } else {
-        a.s1c = a.s2c = a.m2s = 0.f;
+    a.inv_s = inv_s;
+    a.cst = cst;
+    const float is2 = inv_s * inv_s;
+    a.cst2 = cst * is2;
+    a.kz = a.kq = a.kq3 = 0.f;
+    if (MODEL > 0) {
+        const float s1 = cst * inv_s;            // d psf / d s = s1 [u f]
+        const float s2 = -2.0f * inv_s * s1;     // d2 psf / d s^2 = s2 [u f] + s4 [u^3 f]
+        const float s4 = cst * (is2 * is2);
+        a.kz = MODEL == 3 ? s1 * ds : s1;
+        a.kq = MODEL == 3 ? fmaf(s2, ds * ds, s1 * d2s) : s2;
+        a.kq3 = MODEL == 3 ? s4 * (ds * ds) : s4;
     }
     return a;
 }
 
 // Table entries of consecutive pixel indices along one axis.  Neighbouring
-// pixels share an edge: the exp at the upper edge of pixel t is the exp at the
-// lower edge of pixel t+1 (both arguments are the same float, (t + 1/2) - c),
-// and the erf at the upper edge, ((t - c) + 1/2) * sq, is reused as the lower
-// edge of t+1, ((t + 1 - c) - 1/2) * sq, whenever the two arguments are equal
-// (always, unless t - c rounds; then the lower edge is evaluated).  A run of
-// pixels costs about one erf and one exp per pixel instead of two of each.
+// pixels share an edge, so a run of pixels costs one erf and one exp per pixel
+// instead of two of each, and every entry is a difference of edge values.  With
+// u = (t + 1/2) - c at the upper edge of pixel t and f = exp(-u^2 / (2 s^2)) an
+// edge's values are erf / 2, f, u f and, for the widths, u^3 f.  (The reference
+// rounds u as (t - c) + 1/2 inside erf and the width's products, src/gausslib/
+// baselibrary.jl:8-52: the same number to an ulp.)  The one-thread kernels are
+// bound by issue and fixed-latency waits (issue slots 58-66 % busy, FMA pipe
+// 53-59 %), and the tables were a quarter of their instructions: both edges'
+// products per pixel, with the reference's two roundings of u told apart at run
+// time, took 31 per entry (43 with the width's); sharing them takes 21 (28).
+// With the Poisson terms' and Hessian terms' shorter forms: XYNB 11x11 Poisson,
+// 10^6 ROIs, 1909 -> 1644 us; XYNBS 13x13 sCMOS, 10^6, 3533 -> 3103; astigmatic
+// 15x15 Poisson, 300 000, 1436 -> 1207.
 struct EdgeWalk {
-    float ua;    // erf-argument offset (t - c) + 1/2 of the previous pixel's upper edge
-    float erfa;  // erf(ua * sq)
-    float ea;    // exp-argument offset (t + 1/2) - c of the previous pixel's upper edge
-    float fa;    // exp at the previous pixel's upper edge
+    float pos;       // the last edge's position (t + 1/2)
+    float h, f;      // erf / 2 and exp there
+    float g, g3;     // u f, u^3 f
 };
 
+template <bool SIG>
+__device__ __forceinline__ void walk_edge(const Axis &a, EdgeWalk &w)
+{
+    const float u = w.pos - a.c;
+    const float t = u * a.inv_s;
+    w.f = gauss_edge(t);
+    w.h = half_erf(t, w.f);
+    // (rounded products: which of an entry's differences the compiler would
+    // contract into FMAs could differ between the plain and the table kernels,
+    // whose results are the same bits)
+    w.g = __fmul_rn(u, w.f);
+    if (SIG) w.g3 = __fmul_rn(w.g, __fmul_rn(u, u));
+}
+
 // Start a walk at pixel t0: the values of its lower edge.
+template <bool SIG>
 __device__ __forceinline__ EdgeWalk walk_start(int t0, const Axis &a)
 {
-    const float tf = (float)t0;
-    const float ub = __fadd_rn(tf - a.c, -0.5f);
-    const float eb = __fadd_rn(tf, -0.5f) - a.c;
     EdgeWalk w;
-    w.ua = ub;
-    w.ea = eb;
-    w.fa = gauss_edge(eb * a.inv_s);
-    w.erfa = erf_from_gauss(__fmul_rn(ub, a.sq), w.fa);
+    w.pos = (float)t0 - 0.5f;
+    w.g3 = 0.f;
+    walk_edge<SIG>(a, w);
     return w;
 }
 
-// psf: integral_gaussian_1d (baselibrary.jl:8-14); d1, d2:
-// derivative_integral_gaussian_1d (baselibrary.jl:21-33) and s1, s2:
-// derivative_integral_gaussian_1d_sigma (baselibrary.jl:40-52), each without
-// the factor PSF of the other axis.  The expressions keep the reference's
-// association: (t - c) + 1/2 inside erf and the sigma products, (t + 1/2) - c
-// inside exp.
-//
-// VOTE (one-thread-per-ROI kernel only, where a warp's 32 lanes walk in step):
-// the rare re-evaluation of the lower edge's erf sits behind a warp vote, so
-// that it costs issue slots only in the warps that need it.  Measured per
-// kernel (plain launches, sCMOS ADU): astigmatic 15x15 1.874 -> 1.815 ms for
-// 300 000 ROIs, XYNB 7x7 0.153 -> 0.151 ms for 100 000; slower for
-// XYNBSXSY 13x13 (1.331 -> 1.382 ms), XYNB 11x11 (1.791 -> 1.804 ms) and the
-// astigmatic 15x15 Poisson kernel.
-template <bool SIG, bool SECOND, bool VOTE = false>
-__device__ __forceinline__ void walk_entry(int t, const Axis &a, EdgeWalk &w, float &psf,
-                                           float &d1, float &d2, float &s1, float &s2)
+// The next pixel's entry: psf (integral_gaussian_1d, baselibrary.jl:8-14), its
+// derivatives d1, d2 by the position and z1, zq by the width's parameter, each
+// without the factor PSF of the other axis.
+template <bool SIG, bool SECOND>
+__device__ __forceinline__ void walk_entry(const Axis &a, EdgeWalk &w, float &psf, float &d1,
+                                           float &d2, float &z1, float &zq)
 {
-    const float tf = (float)t;
-    const float tc = tf - a.c;
-    const float ua = __fadd_rn(tc, 0.5f), ub = __fadd_rn(tc, -0.5f);
-    // the lower edge's exp argument (t - 1/2) - c is the previous upper edge's
-    // ((t - 1) + 1/2) - c: the same two operands, the same float
-    const float ea = __fadd_rn(tf, 0.5f) - a.c, eb = w.ea;
-    const float fb = w.fa;
-    const float fa = gauss_edge(ea * a.inv_s);
-    float erfb = w.erfa;
-    if (VOTE) {
-        if (__any_sync(0xffffffffu, ub != w.ua)) {
-            const float r = erf_from_gauss(__fmul_rn(ub, a.sq), fb);
-            erfb = ub != w.ua ? r : erfb;
-        }
-    } else if (ub != w.ua) {
-        erfb = erf_from_gauss(__fmul_rn(ub, a.sq), fb);
-    }
-    const float erfa = erf_from_gauss(__fmul_rn(ua, a.sq), fa);
-    // the true value is >= 0 (erf is increasing and ua > ub), so is the
-    // reference's; a negative rounding residue of the tails is cut to 0
-    psf = fmaxf(0.5f * (erfa - erfb), 0.0f);
-    d1 = a.cst * (fa - fb);
-    if (SECOND) d2 = a.cst2 * (ea * fa - eb * fb);
+    const EdgeWalk b = w;  // the lower edge
+    w.pos = b.pos + 1.0f;
+    walk_edge<SIG && SECOND>(a, w);
+    // the true value is >= 0 (erf is increasing), so is the reference's; a
+    // negative rounding residue of the tails is cut to 0
+    psf = fmaxf(w.h - b.h, 0.0f);
+    d1 = a.cst * (w.f - b.f);
+    const float dg = w.g - b.g;
+    if (SECOND) d2 = a.cst2 * dg;
     if (SIG) {
-        s1 = a.s1c * (fa * ua - fb * ub);
-        if (SECOND) s2 = a.s2c * (fa * (ua * ua * ua) - fb * (ub * ub * ub));
+        z1 = a.kz * dg;
+        if (SECOND) zq = fmaf(a.kq3, w.g3 - b.g3, a.kq * dg);
     }
-    w.ua = ua;
-    w.erfa = erfa;
-    w.ea = ea;
-    w.fa = fa;
 }
 
 // Astigmatic width model, src/psf_derivatives.jl:118-163 (per iteration, scalar):
@@ -1162,15 +1150,16 @@ template <int MODEL> struct Slots {
 
 // Likelihood terms of one pixel: compute_likelihood_terms, Poisson
 // src/camera_models.jl:19-34 and sCMOS :36-42 (1/x by rcp_approx, 1 ulp).
+// Poisson: d / mu - 1 with one rounding, and d / mu^2 = (cf + 1) / mu from it.
 template <bool SCMOS>
 __device__ __forceinline__ void likelihood_terms(float d, float v, float mu, float &cf, float &df)
 {
     if (!SCMOS) {
         const float rm = rcp_approx(mu);
-        const float q = d * rm;
+        const float c = fmaf(d, rm, -1.0f);
         const bool pos = mu > 0.01f;
-        cf = pos ? fminf(q - 1.0f, 1e4f) : 0.f;
-        df = pos ? fminf(q * rm, 1e4f) : 0.f;
+        cf = pos ? fminf(c, 1e4f) : 0.f;
+        df = pos ? fminf(fmaf(c, rm, rm), 1e4f) : 0.f;
     } else {
         const float rv = rcp_approx(mu + v);
         cf = (d - mu) * rv;
@@ -1183,9 +1172,8 @@ __device__ __forceinline__ void likelihood_terms(float d, float v, float mu, flo
 __device__ __forceinline__ void likelihood_terms_uncapped(float d, float mu, float &cf, float &df)
 {
     const float rm = rcp_approx(mu);
-    const float q = d * rm;
-    cf = q - 1.0f;
-    df = q * rm;
+    cf = fmaf(d, rm, -1.0f);
+    df = fmaf(cf, rm, rm);
 }
 
 // Whether a Poisson fit's pixel terms need no mu > 0.01 test and no 1e4 cap
@@ -1203,9 +1191,8 @@ __device__ __forceinline__ bool uncapped(float N, float bg, float dmax)
 // sm_100's add/mul/fma .f32x2 take one issue slot for two FP32 operations, each
 // half rounded exactly like the scalar operation.  The one-thread kernel's
 // Newton pixel loop runs rows (t, t+1) of a column as one pair.  Each half
-// evaluates likelihood_terms / _uncapped's expressions with every operation
-// rounded as written, none contracted into an FMA (d - mu as fma(mu, -1, d):
-// one rounding, like the subtraction), as the reference evaluates them.
+// evaluates likelihood_terms / _uncapped's expressions (d - mu as
+// fma(mu, -1, d): one rounding, like the subtraction).
 __device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
 
 template <bool SCMOS, bool UNCAPPED>
@@ -1219,9 +1206,8 @@ __device__ __forceinline__ void likelihood_terms2(float2 d, float2 v, float2 mu,
         df = rv;
     } else {
         const float2 rm = make_float2(rcp_approx(mu.x), rcp_approx(mu.y));
-        const float2 q = __fmul2_rn(d, rm);
-        const float2 c = __fadd2_rn(q, f2(-1.0f));
-        const float2 e = __fmul2_rn(q, rm);
+        const float2 c = __ffma2_rn(d, rm, f2(-1.0f));
+        const float2 e = __ffma2_rn(c, rm, rm);
         if constexpr (UNCAPPED) {
             cf = c;
             df = e;
@@ -1234,55 +1220,41 @@ __device__ __forceinline__ void likelihood_terms2(float2 d, float2 v, float2 mu,
 }
 
 // Column-side contributions to gradient gs and diagonal Hessian hs of one pixel
-// column j with x-table entry (xp, xd1, xd2, xs1, xs2) and the column sums
+// column j with x-table entry (xp, xd1, xd2, z1, zq) and the column sums
 // A = sum_i py cf, B = sum_i py^2 df, E = sum_i cf, F = sum_i df,
-// G = sum_i py ys1 df (dudt and d2udt2 as in src/psf_derivatives.jl).
+// G = sum_i py z1_y df (dudt and d2udt2 as in src/psf_derivatives.jl).
 template <int MODEL, int P>
 __device__ __forceinline__ void col_terms(float (&gs)[P], float (&hs)[P], float xp, float xd1,
-                                          float xd2, float xs1, float xs2, float A, float B,
-                                          float E, float F, float Gc, const Axis &ax,
-                                          const AstigWidths &aw)
+                                          float xd2, float z1, float zq, float A, float B,
+                                          float E, float F, float Gc)
 {
     using S = Slots<MODEL>;
     gs[S::IX] = fmaf(xd1, A, gs[S::IX]);
-    hs[S::IX] += xd2 * A - xd1 * xd1 * B;
+    hs[S::IX] = fmaf(xd2, A, fmaf(-(xd1 * xd1), B, hs[S::IX]));
     gs[S::IN] = fmaf(xp, A, gs[S::IN]);
-    hs[S::IN] -= xp * xp * B;
+    hs[S::IN] = fmaf(-(xp * xp), B, hs[S::IN]);
     gs[S::IB] += E;
     hs[S::IB] -= F;
-    if (MODEL == 1) {
-        gs[4] = fmaf(xs1, A, gs[4]);
-        hs[4] += (ax.m2s * xs1 - xs2) * A - xs1 * xs1 * B - 2.0f * xs1 * xp * Gc;
-    } else if (MODEL == 2) {
-        gs[4] = fmaf(xs1, A, gs[4]);
-        hs[4] += (ax.m2s * xs1 - xs2) * A - xs1 * xs1 * B;
-    } else if (MODEL == 3) {
-        const float c1 = xs1 * aw.dsx;
-        gs[2] = fmaf(c1, A, gs[2]);
-        hs[2] += ((ax.m2s * xs1 - xs2) * (aw.dsx * aw.dsx) + xs1 * aw.d2sx) * A - c1 * c1 * B -
-                 2.0f * c1 * (xp * aw.dsy) * Gc;
+    if (MODEL > 0) {
+        constexpr int K = MODEL == 3 ? 2 : P - 1 < 4 ? P - 1 : 4;
+        gs[K] = fmaf(z1, A, gs[K]);
+        hs[K] = fmaf(zq, A, fmaf(-(z1 * z1), B, hs[K]));
+        if (MODEL != 2) hs[K] = fmaf(-2.0f * z1 * xp, Gc, hs[K]);
     }
 }
 
-// Row-side contributions of pixel row t: y-table entry (yd1, yd2, ys1, ys2) and
-// the row sums C = sum_j xp cf, D = sum_j xp^2 df.
+// Row-side contributions of a pixel row: y-table entry (yd1, yd2, z1, zq) and the
+// row sums C = sum_j xp cf, D = sum_j xp^2 df.
 template <int MODEL, int P>
 __device__ __forceinline__ void row_terms(float (&gs)[P], float (&hs)[P], float yd1, float yd2,
-                                          float ys1, float ys2, float Ct, float Dt,
-                                          const Axis &ay, const AstigWidths &aw)
+                                          float z1, float zq, float Ct, float Dt)
 {
     gs[1] = fmaf(yd1, Ct, gs[1]);
-    hs[1] += yd2 * Ct - yd1 * yd1 * Dt;
-    if (MODEL == 1) {
-        gs[4] = fmaf(ys1, Ct, gs[4]);
-        hs[4] += (ay.m2s * ys1 - ys2) * Ct - ys1 * ys1 * Dt;
-    } else if (MODEL == 2) {
-        gs[5] = fmaf(ys1, Ct, gs[5]);
-        hs[5] += (ay.m2s * ys1 - ys2) * Ct - ys1 * ys1 * Dt;
-    } else if (MODEL == 3) {
-        const float c2 = ys1 * aw.dsy;
-        gs[2] = fmaf(c2, Ct, gs[2]);
-        hs[2] += ((ay.m2s * ys1 - ys2) * (aw.dsy * aw.dsy) + ys1 * aw.d2sy) * Ct - c2 * c2 * Dt;
+    hs[1] = fmaf(yd2, Ct, fmaf(-(yd1 * yd1), Dt, hs[1]));
+    if (MODEL > 0) {
+        constexpr int K = MODEL == 3 ? 2 : P - 1;
+        gs[K] = fmaf(z1, Ct, gs[K]);
+        hs[K] = fmaf(zq, Ct, fmaf(-(z1 * z1), Dt, hs[K]));
     }
 }
 
@@ -1302,7 +1274,8 @@ __device__ __forceinline__ void newton_step(float (&th)[P], const float (&gs)[P]
 
 // Separable structure of dudt_k = sum_t a_kt(j) * b_kt(i): each parameter has
 // one or two terms, each a column function a (x-axis tables) times a row
-// function b, with b in {0: psf_y, 1: d psf_y/dy, 2: 1, 3: d psf_y/dsigma_y}.
+// function b, with b in {0: psf_y, 1: d psf_y/dy, 2: 1, 3: the derivative z1 by
+// the width's parameter}.
 __host__ __device__ constexpr int term_count(int model, int k)
 {
     return ((model == 1 && k == 4) || (model == 3 && k == 2)) ? 2 : 1;
@@ -1371,7 +1344,7 @@ __device__ __forceinline__ void final_pixel(float d, float v, float mu, float py
 template <int MODEL, int P, int NB>
 __device__ __forceinline__ void fisher_column(float (&Fh)[P][P], float (&Fl)[P][P],
                                               const float (&Q)[NB][NB], float xp, float xd1,
-                                              float xs1, const AstigWidths &aw)
+                                              float z1)
 {
     using S = Slots<MODEL>;
     float av[P][2];
@@ -1379,9 +1352,9 @@ __device__ __forceinline__ void fisher_column(float (&Fh)[P][P], float (&Fl)[P][
     av[S::IY][0] = xp;  av[S::IY][1] = 0.f;
     av[S::IN][0] = xp;  av[S::IN][1] = 0.f;
     av[S::IB][0] = 1.f; av[S::IB][1] = 0.f;
-    if (MODEL == 1) { av[4][0] = xs1; av[4][1] = xp; }
-    if (MODEL == 2) { av[4][0] = xs1; av[4][1] = 0.f; av[5][0] = xp; av[5][1] = 0.f; }
-    if (MODEL == 3) { av[2][0] = xs1 * aw.dsx; av[2][1] = xp * aw.dsy; }
+    if (MODEL == 1) { av[4][0] = z1; av[4][1] = xp; }
+    if (MODEL == 2) { av[4][0] = z1; av[4][1] = 0.f; av[5][0] = xp; av[5][1] = 0.f; }
+    if (MODEL == 3) { av[2][0] = z1; av[2][1] = xp; }
 #pragma unroll
     for (int k = 0; k < P; k++)
 #pragma unroll
@@ -1433,8 +1406,7 @@ __device__ __forceinline__ void lm_pixel(float d, float v, float mu, float py, f
 // One column's contribution to F (upper triangle) and g, in FP32.
 template <int MODEL, int P, int NB>
 __device__ __forceinline__ void lm_column(float (&F)[P][P], float (&g)[P], const float (&Q)[NB][NB],
-                                          const float (&Rs)[NB], float xp, float xd1, float xs1,
-                                          const AstigWidths &aw)
+                                          const float (&Rs)[NB], float xp, float xd1, float z1)
 {
     using S = Slots<MODEL>;
     float av[P][2];
@@ -1442,9 +1414,9 @@ __device__ __forceinline__ void lm_column(float (&F)[P][P], float (&g)[P], const
     av[S::IY][0] = xp;  av[S::IY][1] = 0.f;
     av[S::IN][0] = xp;  av[S::IN][1] = 0.f;
     av[S::IB][0] = 1.f; av[S::IB][1] = 0.f;
-    if (MODEL == 1) { av[4][0] = xs1; av[4][1] = xp; }
-    if (MODEL == 2) { av[4][0] = xs1; av[4][1] = 0.f; av[5][0] = xp; av[5][1] = 0.f; }
-    if (MODEL == 3) { av[2][0] = xs1 * aw.dsx; av[2][1] = xp * aw.dsy; }
+    if (MODEL == 1) { av[4][0] = z1; av[4][1] = xp; }
+    if (MODEL == 2) { av[4][0] = z1; av[4][1] = 0.f; av[5][0] = xp; av[5][1] = 0.f; }
+    if (MODEL == 3) { av[2][0] = z1; av[2][1] = xp; }
 #pragma unroll
     for (int k = 0; k < P; k++) {
 #pragma unroll
@@ -1595,14 +1567,25 @@ __device__ __forceinline__ void write_results_warp(const KernelArgs &a, int64_t 
     }
 }
 
+// Both axes of a pass at parameters th (nk = -1 / sqrt(2 pi)).
 template <int MODEL>
-__device__ __forceinline__ void axis_widths(const float *th, const KernelArgs &a, float &sxw,
-                                            float &syw, AstigWidths &aw)
+__device__ __forceinline__ void make_axes(const float *th, const KernelArgs &a, float nk, Axis &ax,
+                                          Axis &ay)
 {
-    if (MODEL == 0) { sxw = syw = a.psf[0]; }
-    else if (MODEL == 1) { sxw = syw = th[4]; }
-    else if (MODEL == 2) { sxw = th[4]; syw = th[5]; }
-    else { astig_widths(th[2], a.psf, aw); sxw = aw.sx; syw = aw.sy; }
+    using S = Slots<MODEL>;
+    const float c = th[S::IN] * nk;
+    if constexpr (MODEL == 3) {
+        AstigWidths w;
+        astig_widths(th[2], a.psf, w);
+        const float ix = __fdiv_rn(1.0f, w.sx), iy = __fdiv_rn(1.0f, w.sy);
+        ax = make_axis<MODEL>(th[S::IX], ix, c * ix, w.dsx, w.d2sx);
+        ay = make_axis<MODEL>(th[S::IY], iy, c * iy, w.dsy, w.d2sy);
+    } else {
+        const float ix = __fdiv_rn(1.0f, MODEL == 0 ? a.psf[0] : th[4]);
+        const float iy = MODEL == 2 ? __fdiv_rn(1.0f, th[5]) : ix;
+        ax = make_axis<MODEL>(th[S::IX], ix, c * ix, 0.f, 0.f);
+        ay = make_axis<MODEL>(th[S::IY], iy, c * iy, 0.f, 0.f);
+    }
 }
 
 // ---- kernel 1: one thread per ROI ---------------------------------------------
@@ -1626,8 +1609,6 @@ __device__ __forceinline__ void fit_rois_r1(const KernelArgs &a, int64_t roi0, i
     constexpr int PS = 1;  // data plane; sCMOS variance tiles are in tensor memory
     constexpr int NB = SIG ? 4 : 3;
     constexpr int LW = TmemVar<BOX>::LW;
-    // edge walks with the warp-voted erf re-evaluation (walk_entry)
-    constexpr bool VOTE = SCMOS && ((MODEL == 3 && BOX >= 15) || BOX <= 7);
     using S = Slots<MODEL>;
     static_assert(B2 >= P, "a warp's pixel slots stage its results");
 
@@ -1658,6 +1639,7 @@ __device__ __forceinline__ void fit_rois_r1(const KernelArgs &a, int64_t roi0, i
     float thb[PL], stp[PL], gb[PL], Fb[PL][PL], Lb = -INFINITY, lam = 1e-3f;
 #pragma unroll
     for (int k = 0; k < PL; k++) { thb[k] = th[k]; stp[k] = 0.f; }
+    const float nk = -__fdiv_rn(1.0f, a.sqrt2pi);
     for (int it = 0; it <= a.iterations; ++it) {
         const bool final_pass = (it == a.iterations);
         if (LM && it > 0) {
@@ -1668,24 +1650,21 @@ __device__ __forceinline__ void fit_rois_r1(const KernelArgs &a, int64_t roi0, i
                                                                          a.max_step[k])),
                                               a.lower[k], a.upper[k]);
         }
-        float sxw, syw;
-        AstigWidths aw;
-        axis_widths<MODEL>(th, a, sxw, syw, aw);
         const float N = th[S::IN], bg = th[S::IB];
-        const Axis ax = make_axis(th[S::IX], sxw, N, a.sqrt2pi, SIG);
-        const Axis ay = make_axis(th[S::IY], syw, N, a.sqrt2pi, SIG);
+        Axis ax, ay;
+        make_axes<MODEL>(th, a, nk, ax, ay);
         {
-            EdgeWalk wy = walk_start(1, ay);
+            EdgeWalk wy = walk_start<SIG>(1, ay);
 #pragma unroll
             for (int t = 0; t < BOX; t++) {
                 float s1 = 0.f, s2 = 0.f;
-                walk_entry<SIG, true, VOTE>(t + 1, ay, wy, py[t], yd1[t], yd2[t], s1, s2);
+                walk_entry<SIG, true>(ay, wy, py[t], yd1[t], yd2[t], s1, s2);
                 if (SIG) { ys1[t] = s1; ys2[t] = s2; }
             }
         }
-        EdgeWalk wx = walk_start(1, ax);
+        EdgeWalk wx = walk_start<SIG>(1, ax);
         float xp, xd1, xd2, xs1 = 0.f, xs2 = 0.f;
-        walk_entry<SIG, true, VOTE>(1, ax, wx, xp, xd1, xd2, xs1, xs2);
+        walk_entry<SIG, true>(ax, wx, xp, xd1, xd2, xs1, xs2);
 
         if (LM && !final_pass) {
             float llr = 0.f;
@@ -1698,7 +1677,7 @@ __device__ __forceinline__ void fit_rois_r1(const KernelArgs &a, int64_t roi0, i
             }
             for (int j = 1; j <= BOX; j++) {
                 float nxp, nxd1, nxd2, nxs1 = 0.f, nxs2 = 0.f;
-                walk_entry<SIG, false, VOTE>(j + 1, ax, wx, nxp, nxd1, nxd2, nxs1, nxs2);
+                walk_entry<SIG, false>(ax, wx, nxp, nxd1, nxd2, nxs1, nxs2);
                 const float npx = N * xp;
                 const float *col = pix + (j - 1) * BOX * PS;
                 float vv[LW];  // this column's variances, from tensor memory
@@ -1718,7 +1697,7 @@ __device__ __forceinline__ void fit_rois_r1(const KernelArgs &a, int64_t roi0, i
                     lm_pixel<SCMOS, SIG, NB>(d, v, mu, py[t], yd1[t], SIG ? ys1[t] : 0.f, llr, Q,
                                              Rs);
                 }
-                lm_column<MODEL, P, NB>(F, gs, Q, Rs, xp, xd1, xs1, aw);
+                lm_column<MODEL, P, NB>(F, gs, Q, Rs, xp, xd1, xs1);
                 xp = nxp; xd1 = nxd1; xs1 = nxs1;
             }
             if constexpr (LM) lm_update<P>(th, thb, stp, gb, Fb, Lb, lam, it == 0, llr, gs, F);
@@ -1761,7 +1740,7 @@ __device__ __forceinline__ void fit_rois_r1(const KernelArgs &a, int64_t roi0, i
                 for (int j = 1; j <= BOX; j++) {
                     // next column's table entry: independent of this column's pixels
                     float nxp, nxd1, nxd2, nxs1 = 0.f, nxs2 = 0.f;
-                    walk_entry<SIG, true, VOTE>(j + 1, ax, wx, nxp, nxd1, nxd2, nxs1, nxs2);
+                    walk_entry<SIG, true>(ax, wx, nxp, nxd1, nxd2, nxs1, nxs2);
                     const float2 xpv = f2(xp);
                     const float2 npx = __fmul2_rn(Nv, xpv), xp2 = __fmul2_rn(xpv, xpv);
                     const float *col = pix + (j - 1) * BOX * PS;
@@ -1803,7 +1782,7 @@ __device__ __forceinline__ void fit_rois_r1(const KernelArgs &a, int64_t roi0, i
                         if (CROSS) Gc.x = fmaf(aGl, df, Gc.x);
                     }
                     col_terms<MODEL, P>(gs, hs, xp, xd1, xd2, xs1, xs2, A.x + A.y, B.x + B.y,
-                                        E.x + E.y, F.x + F.y, Gc.x + Gc.y, ax, aw);
+                                        E.x + E.y, F.x + F.y, Gc.x + Gc.y);
                     if (PIPE && j < BOX) {
                         tmem_ld_wait<LW>(nv);
 #pragma unroll
@@ -1827,7 +1806,7 @@ __device__ __forceinline__ void fit_rois_r1(const KernelArgs &a, int64_t roi0, i
                 const float Ct = pr ? ((t & 1) ? CP[t >> 1].y : CP[t >> 1].x) : Cl;
                 const float Dt = pr ? ((t & 1) ? DP[t >> 1].y : DP[t >> 1].x) : Dl;
                 row_terms<MODEL, P>(gs, hs, yd1[t], yd2[t], SIG ? ys1[t] : 0.f,
-                                    SIG ? ys2[t] : 0.f, Ct, Dt, ay, aw);
+                                    SIG ? ys2[t] : 0.f, Ct, Dt);
             }
             newton_step<P>(th, gs, hs, a);
         } else {
@@ -1839,7 +1818,7 @@ __device__ __forceinline__ void fit_rois_r1(const KernelArgs &a, int64_t roi0, i
                 for (int l = 0; l < P; l++) { Fh[k][l] = 0.f; Fl[k][l] = 0.f; }
             for (int j = 1; j <= BOX; j++) {
                 float nxp, nxd1, nxd2, nxs1 = 0.f, nxs2 = 0.f;
-                walk_entry<SIG, false, VOTE>(j + 1, ax, wx, nxp, nxd1, nxd2, nxs1, nxs2);
+                walk_entry<SIG, false>(ax, wx, nxp, nxd1, nxd2, nxs1, nxs2);
                 const float npx = N * xp;
                 const float *col = pix + (j - 1) * BOX * PS;
                 float vv[LW];  // this column's variances, from tensor memory
@@ -1856,7 +1835,7 @@ __device__ __forceinline__ void fit_rois_r1(const KernelArgs &a, int64_t roi0, i
                     const float mu = fmaf(npx, py[t], bg);
                     final_pixel<SCMOS, SIG, NB>(d, v, mu, py[t], yd1[t], SIG ? ys1[t] : 0.f, llr, Q);
                 }
-                fisher_column<MODEL, P, NB>(Fh, Fl, Q, xp, xd1, xs1, aw);
+                fisher_column<MODEL, P, NB>(Fh, Fl, Q, xp, xd1, xs1);
                 xp = nxp; xd1 = nxd1; xs1 = nxs1;
             }
             double Fm[P][P];
@@ -2006,30 +1985,28 @@ __device__ __forceinline__ void fit_rois_tpr(const KernelArgs &a, int64_t roi0, 
         }
     }
 
+    const float nk = -__fdiv_rn(1.0f, a.sqrt2pi);
     for (int it = 0; it <= a.iterations; ++it) {
         const bool final_pass = (it == a.iterations);
-        float sxw, syw;
-        AstigWidths aw;
-        axis_widths<MODEL>(th, a, sxw, syw, aw);
         const float N = th[S::IN], bg = th[S::IB];
-        const Axis ax = make_axis(th[S::IX], sxw, N, a.sqrt2pi, SIG);
-        const Axis ay = make_axis(th[S::IY], syw, N, a.sqrt2pi, SIG);
+        Axis ax, ay;
+        make_axes<MODEL>(th, a, nk, ax, ay);
 
         // this lane's rows of the y tables (slot t: row r0 + t + 1; a slot
         // past the block is evaluated but not used)
         float py[RMAX], yd1[RMAX], yd2[RMAX], ys1[SIG ? RMAX : 1], ys2[SIG ? RMAX : 1];
         {
-            EdgeWalk wy = walk_start(r0 + 1, ay);
+            EdgeWalk wy = walk_start<SIG>(r0 + 1, ay);
 #pragma unroll
             for (int t = 0; t < RMAX; t++) {
                 float s1 = 0.f, s2 = 0.f;
-                walk_entry<SIG, true>(r0 + t + 1, ay, wy, py[t], yd1[t], yd2[t], s1, s2);
+                walk_entry<SIG, true>(ay, wy, py[t], yd1[t], yd2[t], s1, s2);
                 if (SIG) { ys1[t] = s1; ys2[t] = s2; }
             }
         }
-        EdgeWalk wx = walk_start(c0 + 1, ax);
+        EdgeWalk wx = walk_start<SIG>(c0 + 1, ax);
         float xp, xd1, xd2, xs1 = 0.f, xs2 = 0.f;  // the lane's current column
-        walk_entry<SIG, true>(c0 + 1, ax, wx, xp, xd1, xd2, xs1, xs2);
+        walk_entry<SIG, true>(ax, wx, xp, xd1, xd2, xs1, xs2);
 
         if (!final_pass) {
             float py2[RMAX], aG[CROSS ? RMAX : 1], C[RMAX], D[RMAX];
@@ -2048,7 +2025,7 @@ __device__ __forceinline__ void fit_rois_tpr(const KernelArgs &a, int64_t roi0, 
                 for (int j = c0 + 1; j <= c1; j++) {
                     // next column's entry: independent of this column's pixels
                     float nxp, nxd1, nxd2, nxs1 = 0.f, nxs2 = 0.f;
-                    walk_entry<SIG, true>(j + 1, ax, wx, nxp, nxd1, nxd2, nxs1, nxs2);
+                    walk_entry<SIG, true>(ax, wx, nxp, nxd1, nxd2, nxs1, nxs2);
                     const float npx = N * xp, xp2 = xp * xp;
                     const float *col = pix + ((j - 1) * BOX + r0) * PS;
                     float A[2] = {0.f, 0.f}, B[2] = {0.f, 0.f}, E[2] = {0.f, 0.f},
@@ -2077,8 +2054,7 @@ __device__ __forceinline__ void fit_rois_tpr(const KernelArgs &a, int64_t roi0, 
                         if (CROSS) Gc[h] = fmaf(aG[t], df, Gc[h]);
                     }
                     col_terms<MODEL, P>(gs, hs, xp, xd1, xd2, xs1, xs2, A[0] + A[1],
-                                        B[0] + B[1], E[0] + E[1], F[0] + F[1], Gc[0] + Gc[1],
-                                        ax, aw);
+                                        B[0] + B[1], E[0] + E[1], F[0] + F[1], Gc[0] + Gc[1]);
                     xp = nxp; xd1 = nxd1; xd2 = nxd2; xs1 = nxs1; xs2 = nxs2;
                 }
             };
@@ -2094,7 +2070,7 @@ __device__ __forceinline__ void fit_rois_tpr(const KernelArgs &a, int64_t roi0, 
             for (int t = 0; t < RMAX; t++) {
                 if (t == RMAX - 1 && !last_row) break;
                 row_terms<MODEL, P>(gs, hs, yd1[t], yd2[t], SIG ? ys1[t] : 0.f,
-                                    SIG ? ys2[t] : 0.f, C[t], D[t], ay, aw);
+                                    SIG ? ys2[t] : 0.f, C[t], D[t]);
             }
 #pragma unroll
             for (int k = 0; k < P; k++) {
@@ -2111,7 +2087,7 @@ __device__ __forceinline__ void fit_rois_tpr(const KernelArgs &a, int64_t roi0, 
                 for (int l = 0; l < P; l++) { Fh[k][l] = 0.f; Fl[k][l] = 0.f; }
             for (int j = c0 + 1; j <= c1; j++) {
                 float nxp, nxd1, nxd2, nxs1 = 0.f, nxs2 = 0.f;
-                walk_entry<SIG, false>(j + 1, ax, wx, nxp, nxd1, nxd2, nxs1, nxs2);
+                walk_entry<SIG, false>(ax, wx, nxp, nxd1, nxd2, nxs1, nxs2);
                 const float npx = N * xp;
                 const float *col = pix + ((j - 1) * BOX + r0) * PS;
                 float Q[NB][NB];
@@ -2133,7 +2109,7 @@ __device__ __forceinline__ void fit_rois_tpr(const KernelArgs &a, int64_t roi0, 
                     final_pixel<SCMOS, SIG, NB>(d, v, mu, py[t], yd1[t], SIG ? ys1[t] : 0.f,
                                                 llr, Q);
                 }
-                fisher_column<MODEL, P, NB>(Fh, Fl, Q, xp, xd1, xs1, aw);
+                fisher_column<MODEL, P, NB>(Fh, Fl, Q, xp, xd1, xs1);
                 xp = nxp; xd1 = nxd1; xs1 = nxs1;
             }
             llr = group_sum(llr, TPR);

@@ -143,44 +143,28 @@ __device__ __forceinline__ float warp_sum(float v)
     return v;
 }
 
-// One axis of a pass: centre, 1/sigma, -N / (sqrt(2 pi) sigma), and for the
-// astigmatic model the width's derivatives with respect to z.
-struct WarpAxis {
-    float c, is, cst, ds, d2s;
-};
-
 // Table entries of the pixels whose lower edge is e (0-based pixel e, from the
-// lanes' edges e and e + 1): psf, its first and second derivative by the
-// position, and for the fitted widths the first and second derivative by the
-// width's parameter; each without the other axis' psf (walk_entry's values).
+// lanes' edges e and e + 1): walk_entry's values, at tab + k box for k = 0..4.
 // `width` lanes share an axis, edge index = lane within them.
 template <int MODEL>
-__device__ __forceinline__ void warp_entry(int e, const WarpAxis &w, int width, bool keep,
-                                           float *tab, int box)
+__device__ __forceinline__ void warp_entry(int e, const Axis &a, int width, bool keep, float *tab,
+                                           int box)
 {
     constexpr bool SIG = ModelInfo<MODEL>::SIG;
-    const float u = __fadd_rn((float)e, 0.5f) - w.c;
-    const float f = gauss_edge(u * w.is);
-    const float erf = erf_from_gauss(u * (0.70710678118654752f * w.is), f);
-    const float uf = u * f;
-    const float derf = __shfl_down_sync(0xffffffffu, erf, 1, width) - erf;
-    const float df = __shfl_down_sync(0xffffffffu, f, 1, width) - f;
-    const float duf = __shfl_down_sync(0xffffffffu, uf, 1, width) - uf;
-    float du3 = 0.f;
-    if (SIG) {
-        const float u3 = uf * (u * u);
-        du3 = __shfl_down_sync(0xffffffffu, u3, 1, width) - u3;
-    }
+    EdgeWalk w;
+    w.pos = (float)e + 0.5f;
+    w.g3 = 0.f;
+    walk_edge<SIG>(a, w);
+    auto diff = [&](float v) { return __shfl_down_sync(0xffffffffu, v, 1, width) - v; };
+    const float dh = diff(w.h), df = diff(w.f), dg = diff(w.g);
+    const float dg3 = SIG ? diff(w.g3) : 0.f;
     if (keep) {
-        const float is2 = w.is * w.is;
-        tab[e] = fmaxf(0.5f * derf, 0.0f);
-        tab[box + e] = w.cst * df;
-        tab[2 * box + e] = (w.cst * is2) * duf;
+        tab[e] = fmaxf(dh, 0.0f);
+        tab[box + e] = a.cst * df;
+        tab[2 * box + e] = a.cst2 * dg;
         if (SIG) {
-            const float s1 = (w.cst * w.is) * duf;
-            const float q = fmaf(-2.0f * w.is, s1, (w.cst * (is2 * is2)) * du3);
-            tab[3 * box + e] = MODEL == 3 ? s1 * w.ds : s1;
-            tab[4 * box + e] = MODEL == 3 ? fmaf(q, w.ds * w.ds, s1 * w.d2s) : q;
+            tab[3 * box + e] = a.kz * dg;
+            tab[4 * box + e] = fmaf(a.kq3, dg3, a.kq * dg);
         }
     }
 }
@@ -427,31 +411,28 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
 
     for (int it = 0; it <= a.iterations; ++it) {
         const float N = th[S::IN], bg = th[S::IB];
-        WarpAxis w;
-        w.c = half ? th[1] : th[0];
-        w.ds = w.d2s = 0.f;
-        float s;
-        if (MODEL == 0) s = a.psf[0];
-        else if (MODEL == 1) s = th[4];
-        else if (MODEL == 2) s = half ? th[P - 1] : th[4];
+        // this lane's axis: centre, 1/sigma, -N / (sqrt(2 pi) sigma) and, for the
+        // astigmatic model, the width's derivatives by z
+        const float centre = half ? th[1] : th[0];
+        float sigma, ds = 0.f, d2s = 0.f;
+        if (MODEL == 0) sigma = a.psf[0];
+        else if (MODEL == 1) sigma = th[4];
+        else if (MODEL == 2) sigma = half ? th[P - 1] : th[4];
         else
             astig_width(th[2], half ? a.psf[6] : -a.psf[6], half ? a.psf[1] : a.psf[0],
-                        half ? a.psf[3] : a.psf[2], half ? a.psf[5] : a.psf[4], a.psf[7], s,
-                        w.ds, w.d2s);
-        w.is = __fdiv_rn(1.0f, s);
-        w.cst = N * nk * w.is;
+                        half ? a.psf[3] : a.psf[2], half ? a.psf[5] : a.psf[4], a.psf[7], sigma,
+                        ds, d2s);
+        const float is = __fdiv_rn(1.0f, sigma), cst = N * nk * is;
         __syncwarp();  // the previous pass has read the tables
         if (RMAX <= 4 && box <= 15) {  // both axes at once, at most 16 edges each
             const int e = lane & 15;
-            warp_entry<MODEL>(e, w, 16, e < box, half ? ytab : tab, box);
+            warp_entry<MODEL>(e, make_axis<MODEL>(centre, is, cst, ds, d2s), 16, e < box,
+                              half ? ytab : tab, box);
         } else {
             for (int axis = 0; axis < 2; axis++) {
-                WarpAxis u;
-                u.c = __shfl_sync(0xffffffffu, w.c, 16 * axis);
-                u.is = __shfl_sync(0xffffffffu, w.is, 16 * axis);
-                u.cst = __shfl_sync(0xffffffffu, w.cst, 16 * axis);
-                u.ds = MODEL == 3 ? __shfl_sync(0xffffffffu, w.ds, 16 * axis) : 0.f;
-                u.d2s = MODEL == 3 ? __shfl_sync(0xffffffffu, w.d2s, 16 * axis) : 0.f;
+                auto of = [&](float v) { return __shfl_sync(0xffffffffu, v, 16 * axis); };
+                const Axis u = make_axis<MODEL>(of(centre), of(is), of(cst), MODEL == 3 ? of(ds) : 0.f,
+                                                MODEL == 3 ? of(d2s) : 0.f);
                 for (int e0 = 0; e0 < box; e0 += 31) {
                     const int e = e0 + lane;
                     warp_entry<MODEL>(e, u, 32, lane < 31 && e < box, axis ? ytab : tab, box);
@@ -533,17 +514,16 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
                 // col_terms with the width's entries already per parameter
                 const float As = A.x + A.y, Bs = B.x + B.y;
                 gh[S::IX][0] = fmaf(xd1, As, gh[S::IX][0]);
-                gh[S::IX][1] += xd2 * As - xd1 * xd1 * Bs;
+                gh[S::IX][1] = fmaf(xd2, As, fmaf(-(xd1 * xd1), Bs, gh[S::IX][1]));
                 gh[S::IN][0] = fmaf(xp, As, gh[S::IN][0]);
-                gh[S::IN][1] -= xp2.x * Bs;
+                gh[S::IN][1] = fmaf(-xp2.x, Bs, gh[S::IN][1]);
                 gh[S::IB][0] += E.x + E.y;
                 gh[S::IB][1] -= F.x + F.y;
                 if (SIG) {
                     constexpr int K = MODEL == 3 ? 2 : 4;
                     gh[K][0] = fmaf(z1, As, gh[K][0]);
-                    float h = zq * As - z1 * z1 * Bs;
-                    if (CROSS) h -= 2.0f * z1 * xp * (Gc.x + Gc.y);
-                    gh[K][1] += h;
+                    gh[K][1] = fmaf(zq, As, fmaf(-(z1 * z1), Bs, gh[K][1]));
+                    if (CROSS) gh[K][1] = fmaf(-2.0f * z1 * xp, Gc.x + Gc.y, gh[K][1]);
                 }
             };
             auto columns = [&](auto tag) {
@@ -569,12 +549,12 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
                 const float Dt = r < 2 * NPR ? ((r & 1) ? D[r / 2].y : D[r / 2].x) : Dl;
                 const float yd1 = row(1, r), yd2 = row(2, r);
                 gh[1][0] = fmaf(yd1, Ct, gh[1][0]);
-                gh[1][1] += yd2 * Ct - yd1 * yd1 * Dt;
+                gh[1][1] = fmaf(yd2, Ct, fmaf(-(yd1 * yd1), Dt, gh[1][1]));
                 if (SIG) {
                     constexpr int K = MODEL == 3 ? 2 : MODEL == 2 ? P - 1 : 4;
                     const float z1 = row(3, r), zq = row(4, r);
                     gh[K][0] = fmaf(z1, Ct, gh[K][0]);
-                    gh[K][1] += zq * Ct - z1 * z1 * Dt;
+                    gh[K][1] = fmaf(zq, Ct, fmaf(-(z1 * z1), Dt, gh[K][1]));
                 }
             }
 
@@ -597,8 +577,6 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
             for (int k = 0; k < P; k++)
 #pragma unroll
                 for (int l = 0; l < P; l++) { Fh[k][l] = 0.f; Fl[k][l] = 0.f; }
-            AstigWidths one;
-            one.dsx = one.dsy = 1.f;  // the tables hold the derivatives by z
             auto column = [&](int j, const float *d, const float *v) {
                 const float xp = tab[j], xd1 = tab[box + j], z1 = SIG ? tab[3 * box + j] : 0.f;
                 const float npx = N * xp;
@@ -617,7 +595,7 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
                                                     SIG ? ytab[3 * box + i] : 0.f, llr, Q);
                     }
                 }
-                fisher_column<MODEL, P, NB>(Fh, Fl, Q, xp, xd1, z1, one);
+                fisher_column<MODEL, P, NB>(Fh, Fl, Q, xp, xd1, z1);
             };
             if constexpr (W::REG) {
 #pragma unroll

@@ -3,7 +3,7 @@
 //
 // The fit evaluates erf and exp at every pixel edge of every iteration, a
 // reciprocal at every pixel and, in the Poisson final pass, two logarithms per
-// pixel (gmle_fit_kernel.cuh: erf_from_gauss, gauss_edge, rcp_approx,
+// pixel (gmle_fit_kernel.cuh: half_erf, gauss_edge, rcp_approx,
 // log_approx).  This entry point evaluates them on caller-supplied arguments
 // next to the CUDA library's erff, expf, IEEE division and logf, in the same
 // kernel, so that a test can bound their error against those and against an
@@ -20,10 +20,10 @@ __global__ void math_selftest_kernel(const float *__restrict__ x, int64_t n, flo
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float v = x[i];
-    // the fit's erf takes exp(-v^2) from gauss_edge at the same edge, whose
-    // argument is the edge offset over sigma (here sqrt(2) v)
-    const float e = gmle::gauss_edge(v * 1.41421356237309515f);
-    out[i] = gmle::erf_from_gauss(v, e);
+    // the fit's erf takes the edge offset over sigma (here sqrt(2) v) and the
+    // exponential of the same edge
+    const float t = v * 1.41421356237309515f;
+    out[i] = 2.0f * gmle::half_erf(t, gmle::gauss_edge(t));
     out[n + i] = erff(v);
     out[2 * n + i] = gmle::gauss_edge(v);
     out[3 * n + i] = expf(-0.5f * (v * v));

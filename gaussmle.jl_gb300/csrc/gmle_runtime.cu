@@ -667,6 +667,7 @@ namespace {
 
 void free_table(TableBufs &b)
 {
+    if (!b.h_base && !b.d_base && !b.d_counter && !b.reuse) return;  // never used
     if (b.reuse) cudaEventSynchronize(b.reuse);
     cudaFreeHost(b.h_base);
     cudaFree(b.d_base);
