@@ -96,6 +96,8 @@ __device__ __forceinline__ float jl_maxf(float x, float y)
     if (isnan(x) || isnan(y)) return x + y;
     return signbit(x - y) ? y : x;
 }
+// jl_maxf(0, x), NaN included
+__device__ __forceinline__ float jl_max0(float x) { return !(x <= 0.f) ? x : 0.f; }
 __device__ __forceinline__ double jl_maxd(double x, double y)
 {
     if (isnan(x) || isnan(y)) return x + y;
@@ -388,7 +390,7 @@ __device__ __forceinline__ void initialize_box(const int BOX, Roi roi, const flo
     float total = 0.f, xw = 0.f, yw = 0.f;
     for (int j = 1; j <= BOX; j++)
         for (int i = 1; i <= BOX; i++) {
-            const float sig = jl_maxf(0.f, __fadd_rn(roi((i - 1) + BOX * (j - 1)), -bg));
+            const float sig = jl_max0(__fadd_rn(roi((i - 1) + BOX * (j - 1)), -bg));
             total = __fadd_rn(total, sig);
             xw = __fadd_rn(xw, __fmul_rn(sig, (float)j));
             yw = __fadd_rn(yw, __fmul_rn(sig, (float)i));
@@ -406,7 +408,7 @@ __device__ __forceinline__ void initialize_box(const int BOX, Roi roi, const flo
         float tot2 = 0.f, mxx = 0.f, myy = 0.f;
         for (int j = 1; j <= BOX; j++)
             for (int i = 1; i <= BOX; i++) {
-                const float sig = jl_maxf(0.f, __fadd_rn(roi((i - 1) + BOX * (j - 1)), -bg));
+                const float sig = jl_max0(__fadd_rn(roi((i - 1) + BOX * (j - 1)), -bg));
                 tot2 = __fadd_rn(tot2, sig);
                 const float dx = __fadd_rn((float)j, -x), dy = __fadd_rn((float)i, -y);
                 mxx = __fadd_rn(mxx, __fmul_rn(__fmul_rn(sig, dx), dx));
@@ -425,11 +427,10 @@ __device__ __forceinline__ void initialize_box(const int BOX, Roi roi, const flo
     }
 }
 
-template <int MODEL, int BOX, int STRIDE>
+template <int MODEL, int BOX>
 __device__ void initialize(const float *roi_pix, const float *psf, float *th)
 {
-    // roi_pix holds the ROI's pixels STRIDE floats apart (2: (data, variance) pairs)
-    initialize_box<MODEL>(BOX, [&](int p) { return roi_pix[STRIDE * p]; }, psf, th);
+    initialize_box<MODEL>(BOX, [&](int p) { return roi_pix[p]; }, psf, th);
 }
 
 // ---- FP64 CRLB from the Fisher matrix, src/unified_kernel.jl:399-431 --------
@@ -559,19 +560,23 @@ __device__ uint8_t crlb_from_fisher(double (&F)[P][P], float *crlb)
 
 // ---- shared pieces of the two kernels ----------------------------------------
 
-// Shared memory, as arrays over the R ROI slots of a block: pixels (float, or
-// float2 (data in e-, read-noise variance) for sCMOS), for sCMOS the map
-// offset of each ROI's first pixel (int64), and one ok flag per slot.
-//
-// One thread per ROI (tpr == 1) keeps only the data plane in shared memory:
-// with sCMOS data each thread's variance tile lives in its tensor-memory lane
-// (TmemVar below), and its ROI's map offset and ok flag in its registers
-// (stage_r1), so a ROI takes box^2 floats.
+// Shared memory, as arrays over the R ROI slots of a block.  One thread per ROI
+// (tpr == 1): the ROI's pixels and nothing else; with sCMOS data each thread's
+// variance tile lives in its tensor-memory lane (TmemVar below), and its ROI's
+// map offset and ok flag in its registers (stage_r1).  Several lanes per ROI:
+// pixels (and variances), for sCMOS the map offset of each ROI's first pixel
+// (int64), and one ok flag per slot; at the end a ROI's pixel slot holds what its
+// inversion needs (result_floats), or, where that is larger, an array of its own.
+__host__ __device__ constexpr int result_floats(int model)
+{
+    const int p = model == 0 ? 4 : model == 2 ? 6 : 5;
+    return p * (p + 1) + p + 1;  // Fisher matrix (upper triangle, float pairs), theta, LLR
+}
 __host__ __device__ inline size_t smem_bytes(int model, int box, bool scmos, int tpr, int rois)
 {
-    (void)model;
     if (tpr == 1) return (size_t)rois * sizeof(float) * box * box;
-    return (size_t)rois * (sizeof(float) * (size_t)box * box * (scmos ? 2 : 1) +
+    const size_t extra = box * box < result_floats(model) ? result_floats(model) : 0;
+    return (size_t)rois * (sizeof(float) * ((size_t)box * box * (scmos ? 2 : 1) + extra) +
                            (scmos ? sizeof(long long) : 0) + sizeof(int));
 }
 
@@ -799,10 +804,10 @@ __device__ __forceinline__ void tmem_ld_wait(float (&v)[LW])
     }
 }
 
-// ADU -> e- of the staged pixels (PS floats apart), (ADU - offset) * gain
+// ADU -> e- of the staged pixels, (ADU - offset) * gain
 // (src/camera_models.jl:110-113).  The gain and offset gathers (L2-resident
 // maps) of kU pixels are issued before any is used, so that they overlap.
-template <int BOX, int PS>
+template <int BOX>
 __device__ __forceinline__ void adu_to_electrons(const KernelArgs &a, float *spix, const int *sok,
                                                  const long long *sbase, int cnt)
 {
@@ -827,7 +832,7 @@ __device__ __forceinline__ void adu_to_electrons(const KernelArgs &a, float *spi
         for (int u = 0; u < kU; u++) {
             const int e = e0 + u * blockDim.x;
             if (e < cnt && sok[e / B2])
-                spix[PS * e] = __fmul_rn(__fadd_rn(spix[PS * e], -off[u]), gn[u]);
+                spix[e] = __fmul_rn(__fadd_rn(spix[e], -off[u]), gn[u]);
         }
     }
 }
@@ -1102,12 +1107,11 @@ __device__ __forceinline__ bool stage_r1(const KernelArgs &a, float *spix, int64
 // (ADU - offset) * gain (src/camera_models.jl:110-113), with the gain/offset
 // loads batched.
 template <int BOX, bool SCMOS>
-__device__ __forceinline__ void stage_block(const KernelArgs &a, float *spix, int *sok, int R,
-                                            int64_t roi0, int nroi)
+__device__ __forceinline__ void stage_block(const KernelArgs &a, float *spix, float *svar,
+                                            long long *sbase, int *sok, int R, int64_t roi0,
+                                            int nroi)
 {
     constexpr int B2 = BOX * BOX;
-    constexpr int PS = SCMOS ? 2 : 1;  // floats per staged pixel
-    long long *sbase = reinterpret_cast<long long *>(spix + R * B2 * PS);
     for (int g = threadIdx.x; g < R; g += blockDim.x) {
         int ok = g < nroi;
         long long base = 0;
@@ -1120,24 +1124,21 @@ __device__ __forceinline__ void stage_block(const KernelArgs &a, float *spix, in
         sok[g] = ok;
         if (SCMOS) sbase[g] = base;
     }
-    const float *src = a.data + roi0 * B2;
-    const int cnt = nroi * B2;
-    if (!SCMOS) {
-        copy_data_plane<BOX>(spix, src, R, nroi);
-    } else {
+    if (SCMOS) {
         __syncthreads();  // sok, sbase
         // consecutive e walk down a column: contiguous map addresses
         for (int e = threadIdx.x; e < R * B2; e += blockDim.x) {
             const int g = e / B2;
             const int p = e - g * B2, j = p / BOX, i = p - j * BOX;
-            const bool in = e < cnt;
-            const bool okg = in && sok[g];
+            const bool okg = g < nroi && sok[g];
             const long long m = sbase[g] + i + (long long)a.ny * j;
-            cp_async4(spix + 2 * e, in ? src + e : a.data, in ? 4u : 0u);
-            cp_async4(spix + 2 * e + 1, okg ? a.var + m : a.var, okg ? 4u : 0u);
+            cp_async4(svar + e, okg ? a.var + m : a.var, okg ? 4u : 0u);
         }
-        cp_async_wait_all();
-        if (a.adu) adu_to_electrons<BOX, 2>(a, spix, sok, sbase, cnt);
+    }
+    copy_data_plane<BOX>(spix, a.data + roi0 * B2, R, nroi);  // waits for all copies
+    if (SCMOS && a.adu) {
+        __syncthreads();  // other threads' copies
+        adu_to_electrons<BOX>(a, spix, sok, sbase, nroi * B2);
     }
     __syncthreads();
 }
@@ -1622,7 +1623,7 @@ __device__ __forceinline__ void fit_rois_r1(const KernelArgs &a, int64_t roi0, i
     float th[P];
 #pragma unroll
     for (int k = 0; k < P; k++) th[k] = 0.f;
-    initialize<MODEL, BOX, PS>(pix, a.psf, th);
+    initialize<MODEL, BOX>(pix, a.psf, th);
     // Poisson: the ROI's largest pixel (NaN if any pixel is NaN), for uncapped()
     float dmax = 0.f;
     if (!SCMOS && !LM) {
@@ -1908,25 +1909,24 @@ __global__ void __launch_bounds__(128)
 // (2, 4 or 8) of one warp share a ROI as a grid of NCX column blocks by NRY row
 // blocks (2 x 1, 4 x 1, 4 x 2): lane (rx, ry) owns columns
 // [rx BOX / NCX, (rx + 1) BOX / NCX) and rows [ry BOX / NRY, (ry + 1) BOX / NRY)
-// of the ROI, evaluates the edge tables of its own columns and rows only, and
-// sums its own pixels.  The column and row terms of the gradient and Hessian
-// (col_terms, row_terms) and the Fisher column terms (fisher_column) are
-// linear in the per-column and per-row sums, so each lane applies them to its
-// partial sums, and only the 2P gradient and Hessian values (and, once, the
-// Fisher matrix and the log-likelihood) are combined across the lanes, by
-// warp shuffles.  Every lane then takes the same Newton step, so theta stays
-// identical in all of them.  The initial estimate is computed by every lane
-// from the staged ROI, in the reference's order.  As in the one-thread
-// kernel, the next column's table entry is evaluated ahead of the current
-// column's pixels, and whole columns of rows are independent work: a lane
-// alone on its scheduler is bound by these chains' latency, not by issue.
+// of the ROI and sums its own pixels, rows in packed pairs as in the one-thread
+// kernel.  Its columns' edge tables it evaluates alone; its rows' are shared out
+// among the NCX lanes of the same rows and exchanged by shuffles.  The column and
+// row terms of the gradient and Hessian (col_terms, row_terms) and
+// the Fisher column terms (fisher_column) are linear in the per-column and
+// per-row sums, so each lane applies them to its partial sums, and only the 2P
+// gradient and Hessian values (and, once, the Fisher matrix and the
+// log-likelihood) are combined across the lanes, by warp shuffles.  Every lane
+// then takes the same Newton step, so theta stays identical.  The initial
+// estimate is computed by every lane from the staged ROI, in the reference's
+// order.  As in the one-thread kernel, the next column's table entry is
+// evaluated ahead of the current column's pixels: a lane alone on its scheduler
+// is bound by these chains' latency, not by issue.
 //
-// Two column blocks evaluate only the y tables twice; four lanes cut a lane's
-// instructions further but add 79 % to the ROI's total (10 000 XYNB 11x11
-// ROIs: 127 k against 71 k lane instructions per ROI).  Measured at 10 000
-// ROIs: astigmatic 15x15 sCMOS 157 us with two lanes, 234 us with four; XYNB
-// 11x11 Poisson 77, 72 and 73 us with two, four and one, where a fit is
-// bound by the latency of its 21 dependent passes.
+// Measured with four lanes at 10 000 XYNB 11x11 Poisson ROIs (two warps per
+// scheduler, issue slots 53 % busy): 63.5 us with every lane evaluating all y
+// entries, scalar pixels and each warp inverting its own eight ROIs; 51.6 us so.
+// Astigmatic 15x15 sCMOS, 9 000: 121 -> 92 us.
 template <int TPR> struct LaneGrid {
     static_assert(TPR == 2 || TPR == 4 || TPR == 8, "2, 4 or 8 lanes per ROI");
     static constexpr int NCX = TPR == 2 ? 2 : 4;
@@ -1942,16 +1942,25 @@ __device__ __forceinline__ void fit_rois_tpr(const KernelArgs &a, int64_t roi0, 
     constexpr bool SIG = ModelInfo<MODEL>::SIG;
     constexpr bool CROSS = (MODEL == 1 || MODEL == 3);
     constexpr int B2 = BOX * BOX;
-    constexpr int PS = SCMOS ? 2 : 1;
     constexpr int NB = SIG ? 4 : 3;
     constexpr int NCX = LaneGrid<TPR>::NCX, NRY = LaneGrid<TPR>::NRY;
     constexpr int RMAX = (BOX + NRY - 1) / NRY;  // rows of the largest row block
+    constexpr int NPR = RMAX / 2;
+    constexpr bool ODD = (RMAX & 1) != 0;
+    constexpr int YR = (RMAX + NCX - 1) / NCX;   // y entries that a lane evaluates
+    constexpr int RES = result_floats(MODEL);
+    constexpr bool RES_IN_PIX = B2 >= RES;
     using S = Slots<MODEL>;
 
     const int R = blockDim.x / TPR;
-    float *spix = smem;
-    int *sok = reinterpret_cast<int *>(spix + R * B2 * PS + (SCMOS ? 2 * R : 0));
-    stage_block<BOX, SCMOS>(a, spix, sok, R, roi0, nroi);
+    // offsets and flags behind the planes: R is a multiple of 4
+    float *spix = smem, *svar = spix + R * B2;
+    float *sres = RES_IN_PIX ? spix : svar + (SCMOS ? R * B2 : 0);
+    constexpr int RS = RES_IN_PIX ? B2 : RES;  // floats between two ROIs' results
+    float *sofs = svar + (SCMOS ? R * B2 : 0) + (RES_IN_PIX ? 0 : R * RES);
+    long long *sbase = reinterpret_cast<long long *>(sofs);
+    int *sok = reinterpret_cast<int *>(sbase + (SCMOS ? R : 0));
+    stage_block<BOX, SCMOS>(a, spix, svar, sbase, sok, R, roi0, nroi);
 
     const int g = threadIdx.x / TPR;  // ROI slot in the block
     const int r = threadIdx.x - g * TPR;
@@ -1959,64 +1968,75 @@ __device__ __forceinline__ void fit_rois_tpr(const KernelArgs &a, int64_t roi0, 
     const int c0 = (rx * BOX) / NCX, c1 = ((rx + 1) * BOX) / NCX;  // columns [c0, c1)
     const int r0 = (ry * BOX) / NRY;
     const int nr = ((ry + 1) * BOX) / NRY - r0;                     // rows [r0, r0 + nr)
-    if (__all_sync(0xffffffffu, g >= nroi)) return;
-    const bool valid = g < nroi && sok[g];
-    const float *pix = spix + g * B2 * PS;
+    const bool fits = !__all_sync(0xffffffffu, g >= nroi);         // one decision per warp
+    const float *pix = spix + g * B2, *var = svar + g * B2;
     // the lane's last row slot holds a row only when its block is a full RMAX
-    const bool last_row = nr == RMAX;
+    const bool last_row = NRY == 1 || nr == RMAX;
 
     float th[P];
 #pragma unroll
     for (int k = 0; k < P; k++) th[k] = 0.f;
-    initialize<MODEL, BOX, PS>(pix, a.psf, th);
-    // Poisson: the largest pixel of the ROI (NaN if any is NaN), for uncapped()
     float dmax = 0.f;
-    if (!SCMOS) {
-        dmax = -INFINITY;
-        for (int j = c0; j < c1; j++)
-            for (int t = 0; t < nr; t++) {
-                const float d = pix[j * BOX + r0 + t];
-                dmax = (d > dmax || d != d) ? d : dmax;
-            }
+    if (fits) {
+        initialize<MODEL, BOX>(pix, a.psf, th);
+        // Poisson: the largest pixel of the ROI (NaN if any is NaN), for uncapped()
+        if (!SCMOS) {
+            dmax = -INFINITY;
+            for (int j = c0; j < c1; j++)
+                for (int t = 0; t < nr; t++) {
+                    const float d = pix[j * BOX + r0 + t];
+                    dmax = (d > dmax || d != d) ? d : dmax;
+                }
 #pragma unroll
-        for (int off = TPR >> 1; off > 0; off >>= 1) {
-            const float o = __shfl_xor_sync(0xffffffffu, dmax, off);
-            dmax = (o > dmax || o != o) ? o : dmax;
+            for (int off = TPR >> 1; off > 0; off >>= 1) {
+                const float o = __shfl_xor_sync(0xffffffffu, dmax, off);
+                dmax = (o > dmax || o != o) ? o : dmax;
+            }
         }
     }
 
     const float nk = -__fdiv_rn(1.0f, a.sqrt2pi);
-    for (int it = 0; it <= a.iterations; ++it) {
+    for (int it = 0; fits && it <= a.iterations; ++it) {
         const bool final_pass = (it == a.iterations);
         const float N = th[S::IN], bg = th[S::IB];
         Axis ax, ay;
         make_axes<MODEL>(th, a, nk, ax, ay);
 
-        // this lane's rows of the y tables (slot t: row r0 + t + 1; a slot
-        // past the block is evaluated but not used)
-        float py[RMAX], yd1[RMAX], yd2[RMAX], ys1[SIG ? RMAX : 1], ys2[SIG ? RMAX : 1];
+        // this lane's share of its rows' table: row slots rx YR .. of the block
+        // (slots past it are evaluated but not used)
+        float ye[SIG ? 5 : 3][YR];
         {
-            EdgeWalk wy = walk_start<SIG>(r0 + 1, ay);
+            EdgeWalk wy = walk_start<SIG>(r0 + rx * YR + 1, ay);
 #pragma unroll
-            for (int t = 0; t < RMAX; t++) {
-                float s1 = 0.f, s2 = 0.f;
-                walk_entry<SIG, true>(ay, wy, py[t], yd1[t], yd2[t], s1, s2);
-                if (SIG) { ys1[t] = s1; ys2[t] = s2; }
+            for (int t = 0; t < YR; t++) {
+                float z1 = 0.f, zq = 0.f;
+                walk_entry<SIG, true>(ay, wy, ye[0][t], ye[1][t], ye[2][t], z1, zq);
+                if constexpr (SIG) { ye[3][t] = z1; ye[4][t] = zq; }
             }
         }
         EdgeWalk wx = walk_start<SIG>(c0 + 1, ax);
         float xp, xd1, xd2, xs1 = 0.f, xs2 = 0.f;  // the lane's current column
         walk_entry<SIG, true>(ax, wx, xp, xd1, xd2, xs1, xs2);
+        // entry k of the lane's row slot t, from the lane that evaluated it
+        const int rows_of = threadIdx.x & 31 & ~(NCX - 1);  // the first lane of these rows
+        auto row = [&](int k, int t) {
+            return __shfl_sync(0xffffffffu, ye[k][t % YR], rows_of + t / YR);
+        };
 
         if (!final_pass) {
-            float py2[RMAX], aG[CROSS ? RMAX : 1], C[RMAX], D[RMAX];
+            float2 pyP[NPR], py2P[NPR], aGP[CROSS ? NPR : 1], CP[NPR], DP[NPR];
 #pragma unroll
-            for (int t = 0; t < RMAX; t++) {
-                py2[t] = py[t] * py[t];
-                if (CROSS) aG[t] = py[t] * ys1[t];
-                C[t] = 0.f;
-                D[t] = 0.f;
+            for (int k = 0; k < NPR; k++) {
+                pyP[k] = make_float2(row(0, 2 * k), row(0, 2 * k + 1));
+                py2P[k] = __fmul2_rn(pyP[k], pyP[k]);
+                if (CROSS) aGP[k] = __fmul2_rn(pyP[k], make_float2(row(CROSS ? 3 : 0, 2 * k), row(CROSS ? 3 : 0, 2 * k + 1)));
+                CP[k] = f2(0.f);
+                DP[k] = f2(0.f);
             }
+            const float pyl = ODD ? row(0, RMAX - 1) : 0.f, py2l = pyl * pyl;
+            const float aGl = CROSS && ODD ? pyl * row(CROSS ? 3 : 0, RMAX - 1) : 0.f;
+            float Cl = 0.f, Dl = 0.f;
+            const float2 Nv = f2(N), bgv = f2(bg);
             float gs[P], hs[P];
 #pragma unroll
             for (int k = 0; k < P; k++) { gs[k] = 0.f; hs[k] = 0.f; }
@@ -2026,35 +2046,49 @@ __device__ __forceinline__ void fit_rois_tpr(const KernelArgs &a, int64_t roi0, 
                     // next column's entry: independent of this column's pixels
                     float nxp, nxd1, nxd2, nxs1 = 0.f, nxs2 = 0.f;
                     walk_entry<SIG, true>(ax, wx, nxp, nxd1, nxd2, nxs1, nxs2);
-                    const float npx = N * xp, xp2 = xp * xp;
-                    const float *col = pix + ((j - 1) * BOX + r0) * PS;
-                    float A[2] = {0.f, 0.f}, B[2] = {0.f, 0.f}, E[2] = {0.f, 0.f},
-                          F[2] = {0.f, 0.f}, Gc[2] = {0.f, 0.f};
+                    const float2 xpv = f2(xp);
+                    const float2 npx = __fmul2_rn(Nv, xpv), xp2 = __fmul2_rn(xpv, xpv);
+                    const float *col = pix + (j - 1) * BOX + r0, *cv = var + (j - 1) * BOX + r0;
+                    float2 A = f2(0.f), B = f2(0.f), E = f2(0.f), F = f2(0.f), Gc = f2(0.f);
 #pragma unroll
-                    for (int t = 0; t < RMAX; t++) {
-                        if (t == RMAX - 1 && !last_row) break;
-                        float d, v = 0.f;
-                        if (SCMOS) {
-                            const float2 q = reinterpret_cast<const float2 *>(col)[t];
-                            d = q.x; v = q.y;
-                        } else {
-                            d = col[t];
+                    for (int k = 0; k < NPR; k++) {
+                        const int t = 2 * k;
+                        const bool in1 = t + 1 < RMAX - 1 || last_row;
+                        const float2 d = make_float2(col[t], in1 ? col[t + 1] : 0.f);
+                        const float2 v = SCMOS ? make_float2(cv[t], in1 ? cv[t + 1] : 1.f) : f2(0.f);
+                        const float2 mu = __ffma2_rn(npx, pyP[k], bgv);
+                        float2 cf, df;
+                        likelihood_terms2<SCMOS, UNCAPPED>(d, v, mu, cf, df);
+                        if (NRY > 1 && t + 1 == RMAX - 1) {  // a slot past the block
+                            cf.y = in1 ? cf.y : 0.f;
+                            df.y = in1 ? df.y : 0.f;
                         }
-                        const float mu = fmaf(npx, py[t], bg);
-                        float cf, df;
-                        if constexpr (UNCAPPED) likelihood_terms_uncapped(d, mu, cf, df);
-                        else likelihood_terms<SCMOS>(d, v, mu, cf, df);
-                        const int h = t & 1;
-                        A[h] = fmaf(py[t], cf, A[h]);
-                        B[h] = fmaf(py2[t], df, B[h]);
-                        E[h] += cf;
-                        F[h] += df;
-                        C[t] = fmaf(xp, cf, C[t]);
-                        D[t] = fmaf(xp2, df, D[t]);
-                        if (CROSS) Gc[h] = fmaf(aG[t], df, Gc[h]);
+                        A = __ffma2_rn(pyP[k], cf, A);
+                        B = __ffma2_rn(py2P[k], df, B);
+                        E = __fadd2_rn(E, cf);
+                        F = __fadd2_rn(F, df);
+                        CP[k] = __ffma2_rn(xpv, cf, CP[k]);
+                        DP[k] = __ffma2_rn(xp2, df, DP[k]);
+                        if (CROSS) Gc = __ffma2_rn(aGP[k], df, Gc);
                     }
-                    col_terms<MODEL, P>(gs, hs, xp, xd1, xd2, xs1, xs2, A[0] + A[1],
-                                        B[0] + B[1], E[0] + E[1], F[0] + F[1], Gc[0] + Gc[1]);
+                    if constexpr (ODD) {
+                        if (last_row) {
+                            const float d = col[RMAX - 1], v = SCMOS ? cv[RMAX - 1] : 0.f;
+                            const float mu = fmaf(npx.x, pyl, bg);
+                            float cf, df;
+                            if constexpr (UNCAPPED) likelihood_terms_uncapped(d, mu, cf, df);
+                            else likelihood_terms<SCMOS>(d, v, mu, cf, df);
+                            A.x = fmaf(pyl, cf, A.x);
+                            B.x = fmaf(py2l, df, B.x);
+                            E.x += cf;
+                            F.x += df;
+                            Cl = fmaf(xp, cf, Cl);
+                            Dl = fmaf(xp2.x, df, Dl);
+                            if (CROSS) Gc.x = fmaf(aGl, df, Gc.x);
+                        }
+                    }
+                    col_terms<MODEL, P>(gs, hs, xp, xd1, xd2, xs1, xs2, A.x + A.y, B.x + B.y,
+                                        E.x + E.y, F.x + F.y, Gc.x + Gc.y);
                     xp = nxp; xd1 = nxd1; xd2 = nxd2; xs1 = nxs1; xs2 = nxs2;
                 }
             };
@@ -2068,9 +2102,13 @@ __device__ __forceinline__ void fit_rois_tpr(const KernelArgs &a, int64_t roi0, 
             }
 #pragma unroll
             for (int t = 0; t < RMAX; t++) {
-                if (t == RMAX - 1 && !last_row) break;
-                row_terms<MODEL, P>(gs, hs, yd1[t], yd2[t], SIG ? ys1[t] : 0.f,
-                                    SIG ? ys2[t] : 0.f, C[t], D[t]);
+                const bool pr = t < 2 * NPR;
+                const float Ct = pr ? ((t & 1) ? CP[t >> 1].y : CP[t >> 1].x) : Cl;
+                const float Dt = pr ? ((t & 1) ? DP[t >> 1].y : DP[t >> 1].x) : Dl;
+                const float yd1 = row(1, t), yd2 = row(2, t);
+                const float z1 = SIG ? row(SIG ? 3 : 0, t) : 0.f, zq = SIG ? row(SIG ? 4 : 0, t) : 0.f;
+                if (t < RMAX - 1 || last_row)
+                    row_terms<MODEL, P>(gs, hs, yd1, yd2, z1, zq, Ct, Dt);
             }
 #pragma unroll
             for (int k = 0; k < P; k++) {
@@ -2085,11 +2123,18 @@ __device__ __forceinline__ void fit_rois_tpr(const KernelArgs &a, int64_t roi0, 
             for (int k = 0; k < P; k++)
 #pragma unroll
                 for (int l = 0; l < P; l++) { Fh[k][l] = 0.f; Fl[k][l] = 0.f; }
+            float py[RMAX], yd1[RMAX], yz[RMAX];
+#pragma unroll
+            for (int t = 0; t < RMAX; t++) {
+                py[t] = row(0, t);
+                yd1[t] = row(1, t);
+                yz[t] = SIG ? row(SIG ? 3 : 0, t) : 0.f;
+            }
             for (int j = c0 + 1; j <= c1; j++) {
                 float nxp, nxd1, nxd2, nxs1 = 0.f, nxs2 = 0.f;
                 walk_entry<SIG, false>(ax, wx, nxp, nxd1, nxd2, nxs1, nxs2);
                 const float npx = N * xp;
-                const float *col = pix + ((j - 1) * BOX + r0) * PS;
+                const float *col = pix + (j - 1) * BOX + r0, *cv = var + (j - 1) * BOX + r0;
                 float Q[NB][NB];
 #pragma unroll
                 for (int p = 0; p < NB; p++)
@@ -2098,32 +2143,48 @@ __device__ __forceinline__ void fit_rois_tpr(const KernelArgs &a, int64_t roi0, 
 #pragma unroll
                 for (int t = 0; t < RMAX; t++) {
                     if (t == RMAX - 1 && !last_row) break;
-                    float d, v = 0.f;
-                    if (SCMOS) {
-                        const float2 q = reinterpret_cast<const float2 *>(col)[t];
-                        d = q.x; v = q.y;
-                    } else {
-                        d = col[t];
-                    }
-                    const float mu = fmaf(npx, py[t], bg);
-                    final_pixel<SCMOS, SIG, NB>(d, v, mu, py[t], yd1[t], SIG ? ys1[t] : 0.f,
-                                                llr, Q);
+                    final_pixel<SCMOS, SIG, NB>(col[t], SCMOS ? cv[t] : 0.f, fmaf(npx, py[t], bg),
+                                                py[t], yd1[t], yz[t], llr, Q);
                 }
                 fisher_column<MODEL, P, NB>(Fh, Fl, Q, xp, xd1, xs1);
                 xp = nxp; xd1 = nxd1; xs1 = nxs1;
             }
             llr = group_sum(llr, TPR);
-            double Fm[P][P];
+            // every lane of the ROI has read its pixels (the sum above)
+            float *res = sres + g * RS;
+            int q = 0;
 #pragma unroll
             for (int k = 0; k < P; k++)
 #pragma unroll
-                for (int l = k; l < P; l++) {
+                for (int l = k; l < P; l++, q++) {
                     dd_group_sum(Fh[k][l], Fl[k][l], TPR);
-                    Fm[k][l] = dd_to_double(Fh[k][l], Fl[k][l]);
-                    Fm[l][k] = Fm[k][l];
+                    if (r == q % TPR) {
+                        res[2 * q] = Fh[k][l];
+                        res[2 * q + 1] = Fl[k][l];
+                    }
                 }
-            if (r == 0 && g < nroi) write_result<P>(a, roi0 + g, valid, th, Fm, llr);
+            if (r == 0) {
+#pragma unroll
+                for (int k = 0; k < P; k++) res[2 * q + k] = th[k];
+                res[2 * q + P] = llr;
+            }
         }
+    }
+    // One thread per ROI inverts for the whole block: a warp's FP64 instruction
+    // takes as long for one lane as for all.
+    __syncthreads();
+    if (threadIdx.x < nroi) {
+        const float *res = sres + threadIdx.x * RS;
+        double Fm[P][P];
+        int q = 0;
+#pragma unroll
+        for (int k = 0; k < P; k++)
+#pragma unroll
+            for (int l = k; l < P; l++, q++)
+                Fm[k][l] = Fm[l][k] = dd_to_double(res[2 * q], res[2 * q + 1]);
+#pragma unroll
+        for (int k = 0; k < P; k++) th[k] = res[2 * q + k];
+        write_result<P>(a, roi0 + threadIdx.x, sok[threadIdx.x], th, Fm, res[2 * q + P]);
     }
 }
 

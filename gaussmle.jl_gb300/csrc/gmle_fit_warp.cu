@@ -226,7 +226,7 @@ __device__ __forceinline__ void warp_initialize_exact(const int box, Each each, 
     for (int i = 0; i < box; i++) edge = __fadd_rn(edge, scr[last + i]);
     const float bg = __fdiv_rn(edge, (float)(4 * box - 4));
     __syncwarp();
-    each([&](int j, int i, float d) { scr[i + box * j] = jl_maxf(0.f, __fadd_rn(d, -bg)); });
+    each([&](int j, int i, float d) { scr[i + box * j] = jl_max0(__fadd_rn(d, -bg)); });
     __syncwarp();
     // weight 1, column or row (1-based): a + b column + c row
     const float wc = lane == 1 ? 1.f : 0.f, wr = lane >= 2 ? 1.f : 0.f;
@@ -272,7 +272,7 @@ __device__ __forceinline__ void warp_initialize(const int box, Each each, const 
     const float bg = __fdiv_rn(warp_sum(edge), (float)(4 * box - 4));
     float total = 0.f, xw = 0.f, yw = 0.f;
     each([&](int j, int i, float d) {
-        const float sig = jl_maxf(0.f, d - bg);
+        const float sig = jl_max0(d - bg);
         total += sig;
         xw = fmaf(sig, (float)(j + 1), xw);
         yw = fmaf(sig, (float)(i + 1), yw);
@@ -284,7 +284,7 @@ __device__ __forceinline__ void warp_initialize(const int box, Each each, const 
     warp_start_xy<MODEL>(box, total, xw, yw, x, y);
     if (MODEL == 3) {
         each([&](int j, int i, float d) {
-            const float sig = jl_maxf(0.f, d - bg);
+            const float sig = jl_max0(d - bg);
             const float dx = (float)(j + 1) - x, dy = (float)(i + 1) - y;
             mxx = fmaf(sig * dx, dx, mxx);
             myy = fmaf(sig * dy, dy, myy);

@@ -87,11 +87,11 @@ namespace gmle_rt {
 //
 // One thread per ROI does the least work per ROI and wins as soon as the batch
 // gives every SM a few warps; several lanes per ROI shorten a fit's chain of
-// dependent passes when it does not.  Measured over models, boxes 5..16 and
-// cameras (us, 4 lanes / one thread): 5 000 ROIs XYNB 11x11 57 / 78, astigmatic
-// 15x15 115 / 131; 10 000: XYNB 11x11 70 / 78, 11x11 sCMOS 74 / 70, XYNBS 13x13
-// sCMOS 115 / 104; 20 000: XYNB 11x11 121 / 98, XYNBS 13x13 sCMOS 205 / 148;
-// 300 000: 1208 / 610 and 2295 / 1112.  The line is drawn at 80 ROIs per SM.
+// dependent passes when it does not.  Measured (us, 4 lanes / one thread):
+// 9 000 ROIs XYNB 11x11 45 / 60, 11x11 sCMOS 47 / 64, XYNBS 13x13 sCMOS 70 / 88,
+// astigmatic 15x15 sCMOS 92 / 130, 16x16 105 / 141; 12 000: 51 / 60, 57 / 64,
+// 90 / 88, 162 / 131, 205 / 145 (a second wave of blocks for the large boxes).  The
+// line is drawn at 80 ROIs per SM, from 15 pixels on at 64.
 //
 // `together` > 0: the launch is one of several, of `together` ROIs in all, that
 // share the SMs and are waited for together: the slowest launch's chain counts
@@ -103,7 +103,8 @@ namespace gmle_rt {
 // ROI: a pass is then a few hundred cycles instead of over a thousand, and all
 // warps are resident at once.  Measured (us, 4 lanes / 8 lanes / a warp): 200 ROIs
 // XYNB 11x11 45 / 43 / 23, astigmatic 15x15 99 / 72 / 37; 2 400 ROIs 45 / 43 / 31 and
-// 100 / 72 / 54; 3 000 ROIs, in two waves of warps, astigmatic 101 / 90 / 84.
+// 100 / 72 / 54 (4 lanes now: 37 and 68); 3 000 ROIs, in two waves of warps,
+// astigmatic 84.
 //
 // ROIs per block of the one-thread kernel: with sCMOS data 128, whose four warps
 // use their tensor-memory columns fully; Poisson data the block that lets
@@ -115,7 +116,7 @@ namespace gmle_rt {
 Tuning default_tuning(int num_sms, int box, bool scmos, int64_t n, int64_t together)
 {
     const int64_t all = together > 0 ? together : n;
-    const int line = together > 0 ? kSubmissionLine : kPlainLine;
+    const int line = together > 0 ? kSubmissionLine : box >= 15 ? kPlainLineLarge : kPlainLine;
     if (all < (int64_t)(together > 0 ? kWarpTogether : kWarpLine) * num_sms)
         return {32, gmle::warp_rois_per_block(num_sms, box, scmos, all)};
     if (all < (int64_t)line * num_sms) return {4, 32};
