@@ -153,41 +153,50 @@ __device__ __forceinline__ bool accept(float lf, float rl, float half_log_lam, f
     return accept_exactly(lf, a, b, invalpha, us, v, k);
 }
 
-// One Poisson(lf) draw from the words of the pixel's counter blocks 0, 1, ...
-__device__ __forceinline__ float poisson_draw(float lf, uint32_t p, uint32_t rlo, uint32_t rhi,
-                                              uint32_t k0, uint32_t k1)
+// Poisson(lf) for 0 < lf < 10 by inversion from the pixel's first word.  rk[k] is
+// 1/k to nearest: q = lf rk, corrected by its residual, is lf / k to nearest
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990; checked for every mantissa and k = 1..64).
+constexpr int kRecips = 65;
+__device__ __forceinline__ float poisson_inversion(float lf, uint32_t word, const float *rk)
 {
-    if (!(lf > 0.f)) return 0.f;
-    Words w = philox4x32_10(Words{{p, rlo, rhi, 0u}}, k0, k1);
-    if (lf < 10.f) {
-        const float u = to_uniform_f(w.w[0]);
-        float q = expf(-lf), f = q;
-        int k = 0;
-        while (u > f && k < 1000) {
-            k++;
-            q = __fmul_rn(q, __fdiv_rn(lf, (float)k));
-            f = __fadd_rn(f, q);
+    const float u = to_uniform_f(word);
+    float p = expf(-lf), f = p;
+    int k = 0;
+    while (u > f && k < 1000) {
+        k++;
+        const float kf = (float)k;
+        float q;
+        if (k < kRecips) {
+            const float r = rk[k];
+            q = __fmul_rn(lf, r);
+            q = fmaf(fmaf(-kf, q, lf), r, q);
+        } else {
+            q = __fdiv_rn(lf, kf);
         }
-        return (float)k;
+        p = __fmul_rn(p, q);
+        f = __fadd_rn(f, p);
     }
+    return (float)k;
+}
+
+// One PTRS attempt for Poisson(lf), lf >= 10, from two words of the pixel's
+// counter blocks: whether it is accepted, and the count.
+__device__ __forceinline__ bool poisson_attempt(float lf, uint32_t wu, uint32_t wv, float &k)
+{
     const float slam = __fsqrt_rn(lf);
     const float b = __fadd_rn(0.931f, __fmul_rn(2.53f, slam));
     const float a = __fadd_rn(-0.059f, __fmul_rn(0.02483f, b));
-    const float invalpha = __fadd_rn(1.1239f, __fdiv_rn(1.1328f, __fadd_rn(b, -3.4f)));
     const float vr = __fadd_rn(0.9277f, -__fdiv_rn(3.6224f, __fadd_rn(b, -2.0f)));
-    const float rl = rcp_approx(lf), half_log_lam = 0.5f * log_approx(lf);
-    for (int it = 0; it < 10000; it++) {  // two words per attempt, two attempts per block
-        if (it > 0 && (it & 1) == 0) w = philox4x32_10(Words{{p, rlo, rhi, (uint32_t)it >> 1}}, k0, k1);
-        const float u = __fadd_rn(to_uniform_f(it & 1 ? w.w[2] : w.w[0]), -0.5f);
-        const float v = to_uniform_f(it & 1 ? w.w[3] : w.w[1]);
-        const float us = __fadd_rn(0.5f, -fabsf(u));
-        const float k = floorf(__fadd_rn(__fadd_rn(__fmul_rn(__fadd_rn(__fdiv_rn(__fmul_rn(2.0f, a), us),
-                                                                       b), u), lf), 0.43f));
-        if (us >= 0.07f && v <= vr) return k;
-        if (k < 0.f || (us < 0.013f && v > us)) continue;
-        if (accept(lf, rl, half_log_lam, a, b, invalpha, us, v, k)) return k;
-    }
-    return floorf(lf);
+    const float u = __fadd_rn(to_uniform_f(wu), -0.5f);
+    const float v = to_uniform_f(wv);
+    const float us = __fadd_rn(0.5f, -fabsf(u));
+    k = floorf(__fadd_rn(__fadd_rn(__fmul_rn(__fadd_rn(__fdiv_rn(__fmul_rn(2.0f, a), us), b), u), lf),
+                         0.43f));
+    if (us >= 0.07f && v <= vr) return true;
+    if (k < 0.f || (us < 0.013f && v > us)) return false;
+    const float invalpha = __fadd_rn(1.1239f, __fdiv_rn(1.1328f, __fadd_rn(b, -3.4f)));
+    return accept(lf, rcp_approx(lf), 0.5f * log_approx(lf), a, b, invalpha, us, v, k);
 }
 
 // erf-integrated 1-D Gaussian of pixel t (1-based) around c with width s.
@@ -219,11 +228,38 @@ struct SimArgs {
     unsigned long long *bad;
 };
 
+// Append e to a list of `count` entries (growing up from list[0] with dir 1, down
+// from list[0] with dir -1) where `add`; one counter update per warp.
+__device__ __forceinline__ void push(bool add, int e, uint16_t *list, int dir, int *count)
+{
+    const unsigned m = __activemask(), who = __ballot_sync(m, add);
+    if (who == 0) return;
+    const int lane = threadIdx.x & 31, leader = __ffs(who) - 1;
+    int at = 0;
+    if (lane == leader) at = atomicAdd(count, __popc(who));
+    at = __shfl_sync(m, at, leader);
+    if (add) list[dir * (at + __popc(who & ((1u << lane) - 1u)))] = (uint16_t)e;
+}
+
+// A block makes whole ROIs, up to kSimPixels pixels.  A
+// pixel's cost depends on its rate and on how many attempts its draw takes, so
+// that a warp that drew its 32 pixels one by one waited for the slowest
+// branch and the longest rejection run among them.  The block therefore sorts
+// its pixels into two lists, rates below 10 (inversion) and from 10 on (PTRS),
+// works each list off with full warps, and gives the rejected attempts of a
+// round (a quarter) to full warps again in the next.  200 000 11x11 sCMOS ADU
+// ROIs: 773 -> 689 us, every draw the same.
 __global__ void __launch_bounds__(kSimThreads) simulate_kernel(const SimArgs a, int rois_per_block)
 {
     __shared__ float s_ax[kSimMaxRois][2][kSimMaxBox];  // [roi][x, y][pixel]
     __shared__ float s_n[kSimMaxRois], s_bg[kSimMaxRois];
     __shared__ long long s_base[kSimMaxRois];  // map offset of the ROI's first pixel; -1: bad
+    __shared__ float s_val[kSimPixels];        // a pixel's rate, then its count
+    // pixels still to draw: rates from 10 on at the front of a round's list, and
+    // in the first round's, rates below 10 at its end
+    __shared__ uint16_t s_list[2][kSimPixels];
+    __shared__ int s_small, s_large[2];
+    __shared__ float s_rk[kRecips];
     const int box = a.box, b2 = box * box;
     const int64_t k0 = (int64_t)blockIdx.x * rois_per_block;
     const int64_t left = a.n - k0;
@@ -264,33 +300,79 @@ __global__ void __launch_bounds__(kSimThreads) simulate_kernel(const SimArgs a, 
         }
         s_ax[q][ax][t] = integral_1d(t + 1, c, s);
     }
+    for (int k = threadIdx.x; k < kRecips; k += blockDim.x) s_rk[k] = __fdiv_rn(1.0f, (float)k);
+    if (threadIdx.x == 0) s_small = s_large[0] = s_large[1] = 0;
     __syncthreads();
+
     const float qnan = __int_as_float(0x7fc00000);
-    for (int e = threadIdx.x; e < nk * b2; e += blockDim.x) {
-        const int q = e / b2, p = e - q * b2, j = p / box, i = p - j * box;
+    const int cnt = nk * b2;
+    // e / b2 and p / box for the block's pixel numbers (below 2^11) by
+    // multiplication: exact while e b2 and p box stay below 2^32
+    const uint32_t m_b2 = 0xffffffffu / (uint32_t)b2 + 1u, m_box = 0xffffffffu / (uint32_t)box + 1u;
+    auto roi_of = [&](int e) { return b2 == 1 ? e : (int)__umulhi((uint32_t)e, m_b2); };
+    auto col_of = [&](int p) { return box == 1 ? p : (int)__umulhi((uint32_t)p, m_box); };
+    auto words = [&](int e, uint32_t block) {
+        const int q = roi_of(e);
         const int64_t k = k0 + q;
-        float *dst = a.out + k * b2 + p;
-        const long long base = s_base[q];
-        if (base < 0) {
-            *dst = qnan;
-            continue;
-        }
-        // mu = bg + N (psf_y[i] psf_x[j])
+        return philox4x32_10(Words{{(uint32_t)(e - q * b2), (uint32_t)k,
+                                    (uint32_t)((uint64_t)k >> 32), block}}, a.k0, a.k1);
+    };
+    // rates: mu = bg + N (psf_y[i] psf_x[j])
+    for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
+        const int q = roi_of(e), p = e - q * b2, j = col_of(p), i = p - j * box;
         const float mu = __fadd_rn(s_bg[q], __fmul_rn(s_n[q], __fmul_rn(s_ax[q][1][i], s_ax[q][0][j])));
-        const uint32_t rlo = (uint32_t)k, rhi = (uint32_t)((uint64_t)k >> 32);
-        const float cnt = poisson_draw(mu, (uint32_t)p, rlo, rhi, a.k0, a.k1);
-        if (a.camera == GMLE_CAMERA_POISSON) {
-            *dst = cnt;
-            continue;
+        const bool draw = s_base[q] >= 0 && mu > 0.f;
+        s_val[e] = draw ? mu : 0.f;
+        push(draw && mu < 10.f, e, &s_list[0][kSimPixels - 1], -1, &s_small);
+        push(draw && !(mu < 10.f), e, &s_list[0][0], 1, &s_large[0]);
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < s_small; t += blockDim.x) {
+        const int e = s_list[0][kSimPixels - 1 - t];
+        s_val[e] = poisson_inversion(s_val[e], words(e, 0u).w[0], s_rk);
+    }
+    for (int it = 0, cur = 0; it < 10000; it++, cur ^= 1) {
+        const int n = s_large[cur];
+        if (n == 0) break;  // the same for the whole block
+        for (int t = threadIdx.x; t < n; t += blockDim.x) {
+            const int e = s_list[cur][t];
+            // two words per attempt, two attempts per counter block
+            const Words w = words(e, (uint32_t)it >> 1);
+            const float lf = s_val[e];
+            float k;
+            bool ok = poisson_attempt(lf, it & 1 ? w.w[2] : w.w[0], it & 1 ? w.w[3] : w.w[1], k);
+            if (it == 9999 && !ok) {
+                k = floorf(lf);
+                ok = true;
+            }
+            if (ok) s_val[e] = k;
+            push(!ok, e, &s_list[cur ^ 1][0], 1, &s_large[cur ^ 1]);
         }
-        const long long m = base + i + (long long)a.ny * j;
-        const Words w = philox4x32_10(Words{{(uint32_t)p, rlo, rhi, kNoiseBlock}}, a.k0, a.k1);
-        const float u1 = to_uniform_f(w.w[0]), u2 = to_uniform_f(w.w[1]);
-        const float z = __fmul_rn(__fsqrt_rn(__fmul_rn(-2.0f, logf(u1))),
-                                  cosf(__fmul_rn(6.28318530717958648f, u2)));
-        const float tot = __fadd_rn(cnt, __fmul_rn(z, __fsqrt_rn(a.var[m])));
-        *dst = a.camera == GMLE_CAMERA_SCMOS ? tot
-                                             : __fadd_rn(__fdiv_rn(tot, a.gain[m]), a.offset[m]);
+        __syncthreads();
+        if (threadIdx.x == 0) s_large[cur] = 0;
+        __syncthreads();
+    }
+    __syncthreads();
+    // read noise and camera, written coalesced
+    float *dst = a.out + k0 * b2;
+    for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
+        const int q = roi_of(e), p = e - q * b2;
+        const long long base = s_base[q];
+        float v = s_val[e];
+        if (base < 0) {
+            v = qnan;
+        } else if (a.camera != GMLE_CAMERA_POISSON) {
+            const int j = col_of(p), i = p - j * box;
+            const long long m = base + i + (long long)a.ny * j;
+            const Words w = words(e, kNoiseBlock);
+            const float u1 = to_uniform_f(w.w[0]), u2 = to_uniform_f(w.w[1]);
+            const float z = __fmul_rn(__fsqrt_rn(__fmul_rn(-2.0f, logf(u1))),
+                                      cosf(__fmul_rn(6.28318530717958648f, u2)));
+            v = __fadd_rn(v, __fmul_rn(z, __fsqrt_rn(a.var[m])));
+            if (a.camera == GMLE_CAMERA_SCMOS_ADU)
+                v = __fadd_rn(__fdiv_rn(v, a.gain[m]), a.offset[m]);
+        }
+        dst[e] = v;
     }
 }
 
