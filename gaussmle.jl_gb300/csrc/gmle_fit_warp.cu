@@ -25,11 +25,11 @@
 // instruction takes as long for one lane as for all, so the block's ROIs
 // share them.
 //
-// Bound: instruction issue and, at 12 resident warps per SM (147 registers for
+// Bound: instruction issue and, at 16 resident warps per SM (128 registers for
 // 21x21 sCMOS), the latency of a pass (no contraction, operands in registers).
 // 12 000 astigmatic 21x21 sCMOS ADU ROIs: 2281 us with one thread per ROI and
 // the pixels and tables in shared memory (one block of 32 threads per SM),
-// 335 us so.  200 XYNB 11x11 ROIs: 45 us with four lanes per ROI, 23 us so.
+// 278 us so.  200 XYNB 11x11 ROIs: 45 us with four lanes per ROI, 23 us so.
 #if !defined(GMLE_MODEL) || !defined(GMLE_SCMOS)
 #error "compile with -DGMLE_MODEL=<0..3> -DGMLE_SCMOS=<0|1>"
 #endif
@@ -429,6 +429,7 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
             warp_entry<MODEL>(e, make_axis<MODEL>(centre, is, cst, ds, d2s), 16, e < box,
                               half ? ytab : tab, box);
         } else {
+#pragma unroll
             for (int axis = 0; axis < 2; axis++) {
                 auto of = [&](float v) { return __shfl_sync(0xffffffffu, v, 16 * axis); };
                 const Axis u = make_axis<MODEL>(of(centre), of(is), of(cst), MODEL == 3 ? of(ds) : 0.f,
@@ -657,8 +658,14 @@ __device__ __forceinline__ void fit_block_warp(const KernelArgs &a, const int bo
 }
 
 // TABLE as for fit_kernel_r1, with tiles of one ROI per warp (boxes up to 16).
+//
+// Resident blocks: registers are what bounds the warps per SM, and with two or
+// three warps per scheduler the kernel waits more than it issues (54 % of the
+// slots).  Asking for 20 warps (boxes to 16), 16 (to 24) and 12 (beyond) gives
+// 96, 128 and 168 registers without spills: 12 000 astigmatic 21x21 sCMOS ROIs
+// 320 -> 278 us (148 -> 128 registers).
 template <int MODEL, bool SCMOS, int RMAX, bool TABLE>
-__global__ void __launch_bounds__(32 * kWarpMaxRois)
+__global__ void __launch_bounds__(32 * kWarpMaxRois, RMAX <= 4 ? 5 : RMAX <= 6 ? 4 : 3)
     fit_kernel_warp(const KernelArgs a, const TileTable t, const int box)
 {
     extern __shared__ __align__(16) float smem[];
