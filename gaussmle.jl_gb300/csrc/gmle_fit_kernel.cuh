@@ -1735,9 +1735,15 @@ __device__ __forceinline__ void fit_rois_r1(const KernelArgs &a, int64_t roi0, i
             float vv[LW];
             if (PIPE) tmem_ld<LW>(taddr, vv);
             // the column loop, with (UNCAPPED) or without the Poisson terms'
-            // tests and caps
+            // tests and caps; two columns per trip for the large sCMOS boxes,
+            // whose column of variances and next table entry would otherwise be
+            // moved between registers every column (XYNBS 13x13, 10^6 ROIs: 3083
+            // -> 3015 us); the others lose more to the larger loop (XYNB 11x11
+            // Poisson, 10^6: 1630 -> 1656 us; XYNBS 9x9 sCMOS, 200 000: +10 us)
+            constexpr int UNROLL = SCMOS && BOX >= 13 ? 2 : 1;
             auto columns = [&](auto uncapped_tag) {
                 constexpr bool UNCAPPED = decltype(uncapped_tag)::value;
+#pragma unroll UNROLL
                 for (int j = 1; j <= BOX; j++) {
                     // next column's table entry: independent of this column's pixels
                     float nxp, nxd1, nxd2, nxs1 = 0.f, nxs2 = 0.f;
