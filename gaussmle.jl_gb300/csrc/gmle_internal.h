@@ -124,6 +124,7 @@ struct Server;
 struct gmle_ctx {
     int device = 0;
     int num_sms = 0;
+    bool host_pages = false;  // the copy engine reads and writes pageable memory itself
     cudaStream_t s_fit = nullptr, s_h2d = nullptr, s_d2h = nullptr;
     std::string err;
     std::mutex mu;
