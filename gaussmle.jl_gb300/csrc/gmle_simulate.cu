@@ -247,9 +247,11 @@ __device__ __forceinline__ void push(bool add, int e, uint16_t *list, int dir, i
 // branch and the longest rejection run among them.  The block therefore sorts
 // its pixels into two lists, rates below 10 (inversion) and from 10 on (PTRS),
 // works each list off with full warps, and gives the rejected attempts of a
-// round (a quarter) to full warps again in the next.  200 000 11x11 sCMOS ADU
-// ROIs: 773 -> 689 us, every draw the same.
-__global__ void __launch_bounds__(kSimThreads) simulate_kernel(const SimArgs a, int rois_per_block)
+// round (a quarter) to full warps again in the next, twice; the few pixels left
+// then are drawn to the end by a thread each.  200 000 11x11 sCMOS ADU
+// ROIs: 773 -> 621 us, every draw the same.  (Bound: issue, 65 % of the slots busy, at
+// about 700 instructions per pixel and lane, two Philox blocks among them.)
+__global__ void __launch_bounds__(kSimThreads, 5) simulate_kernel(const SimArgs a, int rois_per_block)
 {
     __shared__ float s_ax[kSimMaxRois][2][kSimMaxBox];  // [roi][x, y][pixel]
     __shared__ float s_n[kSimMaxRois], s_bg[kSimMaxRois];
@@ -331,26 +333,36 @@ __global__ void __launch_bounds__(kSimThreads) simulate_kernel(const SimArgs a, 
         const int e = s_list[0][kSimPixels - 1 - t];
         s_val[e] = poisson_inversion(s_val[e], words(e, 0u).w[0], s_rk);
     }
-    for (int it = 0, cur = 0; it < 10000; it++, cur ^= 1) {
-        const int n = s_large[cur];
-        if (n == 0) break;  // the same for the whole block
+    // attempt `it` of pixel e: two words per attempt, two attempts per counter
+    // block; the 10 000th is taken as it comes
+    auto attempt = [&](int e, int it) {
+        const Words w = words(e, (uint32_t)it >> 1);
+        const float lf = s_val[e];
+        float k;
+        bool ok = poisson_attempt(lf, it & 1 ? w.w[2] : w.w[0], it & 1 ? w.w[3] : w.w[1], k);
+        if (it == 9999 && !ok) {
+            k = floorf(lf);
+            ok = true;
+        }
+        if (ok) s_val[e] = k;
+        return ok;
+    };
+    constexpr int kRounds = 2;
+#pragma unroll 1
+    for (int it = 0; it < kRounds; it++) {
+        const int cur = it & 1, n = s_large[cur];
         for (int t = threadIdx.x; t < n; t += blockDim.x) {
             const int e = s_list[cur][t];
-            // two words per attempt, two attempts per counter block
-            const Words w = words(e, (uint32_t)it >> 1);
-            const float lf = s_val[e];
-            float k;
-            bool ok = poisson_attempt(lf, it & 1 ? w.w[2] : w.w[0], it & 1 ? w.w[3] : w.w[1], k);
-            if (it == 9999 && !ok) {
-                k = floorf(lf);
-                ok = true;
-            }
-            if (ok) s_val[e] = k;
-            push(!ok, e, &s_list[cur ^ 1][0], 1, &s_large[cur ^ 1]);
+            push(!attempt(e, it), e, &s_list[cur ^ 1][0], 1, &s_large[cur ^ 1]);
         }
         __syncthreads();
         if (threadIdx.x == 0) s_large[cur] = 0;
         __syncthreads();
+    }
+    for (int t = threadIdx.x; t < s_large[kRounds & 1]; t += blockDim.x) {
+        const int e = s_list[kRounds & 1][t];
+#pragma unroll 1
+        for (int it = kRounds; !attempt(e, it); it++) {}
     }
     __syncthreads();
     // read noise and camera, written coalesced
