@@ -29,7 +29,7 @@
 // 21x21 sCMOS), the latency of a pass (no contraction, operands in registers).
 // 12 000 astigmatic 21x21 sCMOS ADU ROIs: 2281 us with one thread per ROI and
 // the pixels and tables in shared memory (one block of 32 threads per SM),
-// 278 us so.  200 XYNB 11x11 ROIs: 45 us with four lanes per ROI, 23 us so.
+// 270 us so.  200 XYNB 11x11 ROIs: 45 us with four lanes per ROI, 20.5 us so.
 #if !defined(GMLE_MODEL) || !defined(GMLE_SCMOS)
 #error "compile with -DGMLE_MODEL=<0..3> -DGMLE_SCMOS=<0|1>"
 #endif
@@ -48,6 +48,7 @@ constexpr int kCols = 8, kRows = 4;  // the lane grid
 // Rows per lane, RMAX = ceil(box / 4), of the compiled kernels; the row slots
 // from RFULL on may lie outside the smallest box of their range.
 template <int RMAX> struct WarpShape {
+    static constexpr int TS = 4 * RMAX;                   // floats between two tables
     static constexpr bool REG = RMAX <= 8;                // pixels in registers
     static constexpr int CMAX = REG ? (RMAX + 1) / 2 : 1;  // columns per lane, in registers
     static constexpr int RFULL = RMAX == 2 ? 0 : RMAX == 12 ? 8 : RMAX == 16 ? 12 : RMAX - 1;
@@ -57,11 +58,6 @@ template <int RMAX> struct WarpShape {
         return RMAX == 2 ? 0 : (4 * (RMAX - 1) + 1) / kCols;
     }
 };
-__host__ __device__ constexpr int rows_per_lane(int box)
-{
-    return box <= 8 ? 2 : box <= 32 ? (box + 3) / 4 : box <= 48 ? 12 : 16;
-}
-
 template <int P> struct RoiResult {  // what the inversion needs, per ROI of a block
     double F[P * (P + 1) / 2];
     float th[P];
@@ -144,11 +140,10 @@ __device__ __forceinline__ float warp_sum(float v)
 }
 
 // Table entries of the pixels whose lower edge is e (0-based pixel e, from the
-// lanes' edges e and e + 1): walk_entry's values, at tab + k box for k = 0..4.
+// lanes' edges e and e + 1): walk_entry's values, at tab + k TS for k = 0..4.
 // `width` lanes share an axis, edge index = lane within them.
-template <int MODEL>
-__device__ __forceinline__ void warp_entry(int e, const Axis &a, int width, bool keep, float *tab,
-                                           int box)
+template <int MODEL, int TS>
+__device__ __forceinline__ void warp_entry(int e, const Axis &a, int width, bool keep, float *tab)
 {
     constexpr bool SIG = ModelInfo<MODEL>::SIG;
     EdgeWalk w;
@@ -160,11 +155,11 @@ __device__ __forceinline__ void warp_entry(int e, const Axis &a, int width, bool
     const float dg3 = SIG ? diff(w.g3) : 0.f;
     if (keep) {
         tab[e] = fmaxf(dh, 0.0f);
-        tab[box + e] = a.cst * df;
-        tab[2 * box + e] = a.cst2 * dg;
+        tab[TS + e] = a.cst * df;
+        tab[2 * TS + e] = a.cst2 * dg;
         if (SIG) {
-            tab[3 * box + e] = a.kz * dg;
-            tab[4 * box + e] = fmaf(a.kq3, dg3, a.kq * dg);
+            tab[3 * TS + e] = a.kz * dg;
+            tab[4 * TS + e] = fmaf(a.kq3, dg3, a.kq * dg);
         }
     }
 }
@@ -205,56 +200,62 @@ __device__ __forceinline__ void warp_start(float x, float y, float total, float 
 }
 
 // The ROI's start point (src/unified_kernel.jl:158-255) with every sum in the
-// reference's order (initialize_box), bit for bit.  `scr` holds the ROI's pixels;
-// each lane turns its own into photons above the background, then lanes 0, 1
-// and 2 add the plain, column- and row-weighted sums.
+// reference's order (initialize_box), bit for bit.  The lanes write the terms of
+// the sums in that order into `scr` (three arrays of warp_scratch(box) floats, 16-byte
+// aligned, zeros behind the last term), then add them: every lane the edge pixels,
+// lane 0, 1 and 2 the plain, column- and row-weighted sums.
+__device__ __forceinline__ float ordered_sum(const float *v, int n4)
+{
+    float acc = 0.f;
+#pragma unroll 4
+    for (int q = 0; q < n4; q++) {
+        const float4 t = reinterpret_cast<const float4 *>(v)[q];
+        acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, t.x), t.y), t.z), t.w);
+    }
+    return acc;
+}
 template <int MODEL, typename Each>
 __device__ __forceinline__ void warp_initialize_exact(const int box, Each each, float *scr, int lane,
                                                       const float *psf,
                                                       float (&th)[ModelInfo<MODEL>::P])
 {
-    const int last = box * (box - 1);
-    float edge = 0.f;
-#pragma unroll 4
-    for (int i = 0; i < box; i++) edge = __fadd_rn(edge, scr[i]);
-#pragma unroll 4
-    for (int j = 1; j < box - 1; j++) {
-        edge = __fadd_rn(edge, scr[box * j]);
-        edge = __fadd_rn(edge, scr[box * j + box - 1]);
-    }
-#pragma unroll 4
-    for (int i = 0; i < box; i++) edge = __fadd_rn(edge, scr[last + i]);
-    const float bg = __fdiv_rn(edge, (float)(4 * box - 4));
+    const int B2 = box * box, BP = warp_scratch(box);
+    each([&](int j, int i, float d) {  // 4 box - 4 edge pixels, column by column
+        const int e = j == 0 ? i : j == box - 1 ? 3 * box - 4 + i : box + 2 * (j - 1) + (i ? 1 : 0);
+        if (j == 0 || j == box - 1 || i == 0 || i == box - 1) scr[e] = d;
+    });
     __syncwarp();
-    each([&](int j, int i, float d) { scr[i + box * j] = jl_max0(__fadd_rn(d, -bg)); });
+    const float bg = __fdiv_rn(ordered_sum(scr, box - 1), (float)(4 * box - 4));
     __syncwarp();
-    // weight 1, column or row (1-based): a + b column + c row
-    const float wc = lane == 1 ? 1.f : 0.f, wr = lane >= 2 ? 1.f : 0.f;
-    const float w0 = lane == 0 ? 1.f : 0.f;
-    float acc = 0.f;
-    for (int j = 0; j < box; j++) {
-        float w = wc * (float)(j + 1) + w0 + wr;  // row 1's weight
-#pragma unroll 4
-        for (int i = 0; i < box; i++) {
-            acc = __fadd_rn(acc, __fmul_rn(scr[i + box * j], w));
-            w += wr;
-        }
-    }
+    each([&](int j, int i, float d) {
+        const float sig = jl_max0(__fadd_rn(d, -bg));
+        float *t = scr + i + box * j;
+        t[0] = sig;
+        t[BP] = __fmul_rn(sig, (float)(j + 1));
+        t[2 * BP] = __fmul_rn(sig, (float)(i + 1));
+    });
+    const int own = min(lane, 2) * BP;
+    if (lane < 3)
+        for (int p = B2; p < BP; p++) scr[own + p] = 0.f;
+    __syncwarp();
+    const float acc = ordered_sum(scr + own, BP / 4);
     const float total = __shfl_sync(0xffffffffu, acc, 0);
     float x, y, mxx = 0.f, myy = 0.f;
     warp_start_xy<MODEL>(box, total, __shfl_sync(0xffffffffu, acc, 1),
                          __shfl_sync(0xffffffffu, acc, 2), x, y);
-    if (MODEL == 3) {  // lane 0: about x, the others: about y
-        acc = 0.f;
-        for (int j = 0; j < box; j++)
-#pragma unroll 4
-            for (int i = 0; i < box; i++) {
-                const float d = lane == 0 ? __fadd_rn((float)(j + 1), -x)
-                                          : __fadd_rn((float)(i + 1), -y);
-                acc = __fadd_rn(acc, __fmul_rn(__fmul_rn(scr[i + box * j], d), d));
-            }
-        mxx = __shfl_sync(0xffffffffu, acc, 0);
-        myy = __shfl_sync(0xffffffffu, acc, 1);
+    if (MODEL == 3) {  // lane 0: about x, lane 1: about y
+        __syncwarp();
+        each([&](int j, int i, float d) {
+            const float sig = jl_max0(__fadd_rn(d, -bg));
+            const float dx = __fadd_rn((float)(j + 1), -x), dy = __fadd_rn((float)(i + 1), -y);
+            float *t = scr + i + box * j;
+            t[0] = __fmul_rn(__fmul_rn(sig, dx), dx);
+            t[BP] = __fmul_rn(__fmul_rn(sig, dy), dy);
+        });
+        __syncwarp();
+        const float m = ordered_sum(scr + min(lane, 1) * BP, BP / 4);
+        mxx = __shfl_sync(0xffffffffu, m, 0);
+        myy = __shfl_sync(0xffffffffu, m, 1);
     }
     warp_start<MODEL>(x, y, total, bg, mxx, myy, psf, th);
 }
@@ -312,7 +313,9 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
     const int lane = threadIdx.x & 31;
     const int ry = lane & (kRows - 1), rx = lane / kRows;
     const int B2 = box * box;
-    float *const spix = tab + 10 * box, *const svar = spix + B2;  // (warp_floats)
+    constexpr int TS = W::TS;
+    float *const spix = tab + 10 * TS, *const svar = spix + warp_scratch(box);  // (warp_floats)
+    for (int e = lane; e < 10 * TS; e += 32) tab[e] = 0.f;  // entries past the box
     bool ok = true;
     long long base = 0;
     if (SCMOS) {
@@ -340,7 +343,9 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
 #pragma unroll
             for (int r = 0; r < RM; r++) {
                 const int j = rx + kCols * c, i = ry + kRows * r;
-                float d = 0.f, v = 0.f;
+                // a slot outside the box: with an infinite variance its
+                // likelihood terms are 0
+                float d = 0.f, v = INFINITY;
                 if (j < box && i < box) fetch(j, i, d, v);
                 dp[c][r] = d;
                 if (SCMOS) vp[c][r] = v;
@@ -368,21 +373,19 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
                 for (int i = ry; i < box; i += kRows) fn(j, i, spix[i + box * j]);
         }
     };
-    // column j of the lane's pixels (slots outside the box: 0)
+    // column j of the lane's pixels
     auto load_column = [&](int j) {
 #pragma unroll
         for (int r = 0; r < RM; r++) {
             const int i = ry + kRows * r;
             const bool in = r < W::RFULL || i < box;
             dp[0][r] = in ? spix[i + box * j] : 0.f;
-            if (SCMOS) vp[0][r] = in ? svar[i + box * j] : 0.f;
+            if (SCMOS) vp[0][r] = in ? svar[i + box * j] : INFINITY;
         }
     };
 
     float th[P];
     if constexpr (RMAX <= 4) {
-        each([&](int j, int i, float d) { spix[i + box * j] = d; });
-        __syncwarp();
         warp_initialize_exact<MODEL>(box, each, spix, lane, a.psf, th);
     } else {
         warp_initialize<MODEL>(box, each, a.psf, th);
@@ -407,7 +410,7 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
     const float lo = a.lower[mine], hi = a.upper[mine], most = a.max_step[mine];
     const int half = lane >> 4;  // 0: x axis, 1: y axis
     const float nk = -__fdiv_rn(1.0f, a.sqrt2pi);
-    float *const ytab = tab + 5 * box;
+    float *const ytab = tab + 5 * TS;
 
     for (int it = 0; it <= a.iterations; ++it) {
         const float N = th[S::IN], bg = th[S::IB];
@@ -426,8 +429,8 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
         __syncwarp();  // the previous pass has read the tables
         if (RMAX <= 4 && box <= 15) {  // both axes at once, at most 16 edges each
             const int e = lane & 15;
-            warp_entry<MODEL>(e, make_axis<MODEL>(centre, is, cst, ds, d2s), 16, e < box,
-                              half ? ytab : tab, box);
+            warp_entry<MODEL, TS>(e, make_axis<MODEL>(centre, is, cst, ds, d2s), 16, e < box,
+                                  half ? ytab : tab);
         } else {
 #pragma unroll
             for (int axis = 0; axis < 2; axis++) {
@@ -436,7 +439,7 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
                                                 MODEL == 3 ? of(d2s) : 0.f);
                 for (int e0 = 0; e0 < box; e0 += 31) {
                     const int e = e0 + lane;
-                    warp_entry<MODEL>(e, u, 32, lane < 31 && e < box, axis ? ytab : tab, box);
+                    warp_entry<MODEL, TS>(e, u, 32, lane < 31 && e < box, axis ? ytab : tab);
                 }
             }
         }
@@ -445,10 +448,7 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
         // the lane's rows of psf_y (0 outside the box)
         float2 py[NPR];
         float pyl = 0.f;
-        auto row = [&](int k, int r) {  // table k at the lane's row slot r
-            const int i = ry + kRows * r;
-            return (r < W::RFULL || i < box) ? ytab[k * box + i] : 0.f;
-        };
+        auto row = [&](int k, int r) { return ytab[k * TS + ry + kRows * r]; };  // (0 past the box)
 #pragma unroll
         for (int k = 0; k < NPR; k++) py[k] = make_float2(row(0, 2 * k), row(0, 2 * k + 1));
         if (ODD) pyl = row(0, RM - 1);
@@ -470,8 +470,8 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
 
             auto column = [&](auto uncapped_tag, int j, const float *d, const float *v) {
                 constexpr bool UNCAPPED = decltype(uncapped_tag)::value;
-                const float xp = tab[j], xd1 = tab[box + j], xd2 = tab[2 * box + j];
-                const float z1 = SIG ? tab[3 * box + j] : 0.f, zq = SIG ? tab[4 * box + j] : 0.f;
+                const float xp = tab[j], xd1 = tab[TS + j], xd2 = tab[2 * TS + j];
+                const float z1 = SIG ? tab[3 * TS + j] : 0.f, zq = SIG ? tab[4 * TS + j] : 0.f;
                 const float2 npx = f2(N * xp), xpv = f2(xp), xp2 = f2(xp * xp), bgv = f2(bg);
                 float2 A = f2(0.f), B = f2(0.f), E = f2(0.f), F = f2(0.f), Gc = f2(0.f);
 #pragma unroll
@@ -482,7 +482,7 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
                     likelihood_terms2<SCMOS, UNCAPPED>(
                         make_float2(d[r], d[r + 1]),
                         SCMOS ? make_float2(v[r], v[r + 1]) : f2(0.f), mu, cf, df);
-                    if (r + 1 >= W::RFULL) {  // slots that may lie outside the box
+                    if (!SCMOS && r + 1 >= W::RFULL) {  // slots that may lie outside the box
                         const bool i0 = r < W::RFULL || ry + kRows * r < box;
                         const bool i1 = ry + kRows * (r + 1) < box;
                         cf = make_float2(i0 ? cf.x : 0.f, i1 ? cf.y : 0.f);
@@ -497,7 +497,7 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
                     if (CROSS) Gc = __ffma2_rn(aG[k], df, Gc);
                 }
                 if constexpr (ODD) {
-                    const bool in = RM - 1 < W::RFULL || ry + kRows * (RM - 1) < box;
+                    const bool in = SCMOS || RM - 1 < W::RFULL || ry + kRows * (RM - 1) < box;
                     const float mu = fmaf(npx.x, pyl, bg);
                     float cf, df;
                     if constexpr (UNCAPPED) likelihood_terms_uncapped(d[RM - 1], mu, cf, df);
@@ -579,7 +579,7 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
 #pragma unroll
                 for (int l = 0; l < P; l++) { Fh[k][l] = 0.f; Fl[k][l] = 0.f; }
             auto column = [&](int j, const float *d, const float *v) {
-                const float xp = tab[j], xd1 = tab[box + j], z1 = SIG ? tab[3 * box + j] : 0.f;
+                const float xp = tab[j], xd1 = tab[TS + j], z1 = SIG ? tab[3 * TS + j] : 0.f;
                 const float npx = N * xp;
                 float Q[NB][NB];
 #pragma unroll
@@ -592,8 +592,8 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
                     if (r < W::RFULL || i < box) {
                         const float p = ytab[i];
                         final_pixel<SCMOS, SIG, NB>(d[r], SCMOS ? v[r] : 0.f, fmaf(npx, p, bg),
-                                                    p, ytab[box + i],
-                                                    SIG ? ytab[3 * box + i] : 0.f, llr, Q);
+                                                    p, ytab[TS + i],
+                                                    SIG ? ytab[3 * TS + i] : 0.f, llr, Q);
                     }
                 }
                 fisher_column<MODEL, P, NB>(Fh, Fl, Q, xp, xd1, z1);

@@ -14,12 +14,21 @@ constexpr int kLargeMinBox = 17, kLargeMaxBox = 64;
 
 inline bool large_box(int box) { return box >= kLargeMinBox && box <= kLargeMaxBox; }
 
-// Shared memory, floats per ROI: 10 tables of `box` entries, and the ROI's
-// pixels: up to 16 pixels once, for the start point's sums in the reference's
-// order, and beyond 32, which no longer fit a warp's registers, pixels and variances.
+// Rows per lane, RMAX = ceil(box / 4), of the kernel that takes a box.
+__host__ __device__ constexpr int rows_per_lane(int box)
+{
+    return box <= 8 ? 2 : box <= 32 ? (box + 3) / 4 : box <= 48 ? 12 : 16;
+}
+
+// Shared memory, floats per ROI: 10 tables of 4 RMAX entries (a compile-time
+// stride; the entries past the box stay 0), then up to 16 pixels three arrays of
+// the ROI's pixels, for the start point's sums in the reference's order, and
+// beyond 32, which no longer fit a warp's registers, pixels and variances.
+__host__ __device__ constexpr int warp_scratch(int box) { return (box * box + 3) & ~3; }
 __host__ __device__ constexpr int warp_floats(int box, bool scmos)
 {
-    return 10 * box + (box <= 16 ? box * box : box > 32 ? box * box * (scmos ? 2 : 1) : 0);
+    return 40 * rows_per_lane(box) +
+           (box <= 16 ? 3 * warp_scratch(box) : box > 32 ? warp_scratch(box) * (scmos ? 2 : 1) : 0);
 }
 
 // ROIs (warps) per block, up to four (their FP64 inversions share instructions):
