@@ -873,6 +873,17 @@ gmle_status plan_mixed(gmle_ctx *ctx, const gmle_group *groups, int32_t ngroups,
         L.tiles = tiles;
         plan.launches.push_back(L);
     }
+    // The launches share the SMs, whose blocks are handed out launch by launch:
+    // the longest blocks first, so that the submission ends on short ones.  A
+    // block's time goes with its pixels and the model's terms.
+    auto cost = [](int model, int box) { return box * box * (model == 0 ? 2 : 3); };
+    std::stable_sort(plan.plain.begin(), plan.plain.end(), [&](const gmle_group &x, const gmle_group &y) {
+        return cost(x.desc.model, x.desc.box) > cost(y.desc.model, y.desc.box);
+    });
+    std::stable_sort(plan.launches.begin(), plan.launches.end(),
+                     [&](const TableLaunch &x, const TableLaunch &y) {
+                         return cost(x.model, x.box) > cost(y.model, y.box);
+                     });
     return GMLE_OK;
 }
 
