@@ -54,11 +54,12 @@ constexpr int kServerTableCap = 4096;  // groups (requests) per step and kind
 // Requests of this many ROIs, and of boxes up to 10 pixels, are fitted with one
 // thread per ROI, the others with four lanes: by the request's own size, so that
 // its results do not depend on the step it runs in.  One thread takes half the
-// work per ROI and, for the large boxes, a third longer (astigmatic 15x15: 150 us
-// against 103): 100 000 sCMOS ROIs in 10 requests 786 us with four lanes for all
-// boxes above 10, 658 us so; in 40 requests 894 and 861; with the line at 1 000
-// ROIs 777, but 18 000 ROIs in 17 requests went from 386 to 485.
-constexpr int64_t kLargeRequest = 4000;
+// work per ROI, but a larger box's fit a third longer (astigmatic 15x15 sCMOS: 129
+// us against 76) until a request fills the GPU by itself.
+// Line at 4 000 / 12 000 ROIs (us): 28 460 sCMOS ROIs in 7 requests 363 / 321,
+// 100 000 in 40 requests 745 / 714, in 10 requests 570 / 630 (with four lanes for
+// every box above 10: 350, 890, 790, before those were made faster).
+constexpr int64_t kLargeRequest = 12000;
 constexpr int kLargeRequestBox = 10;
 constexpr size_t kLatencyRecord = 1 << 20;  // latencies kept for the percentiles
 
