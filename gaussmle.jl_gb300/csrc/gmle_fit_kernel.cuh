@@ -707,6 +707,17 @@ __host__ __device__ constexpr int tmem_var_cols(int box)
     return need <= 32 ? 32 : need <= 64 ? 64 : need <= 128 ? 128 : need <= 256 ? 256 : 512;
 }
 
+// Threads per block of the one-thread sCMOS kernel in large batches: 128, whose
+// four warps use their columns fully, or, where an SM's 228 KiB of shared memory
+// hold only one block of 128 ROIs (16x16), 224, whose fifth to seventh warps take a
+// second set of columns: 200 000 XYNB 16x16 ROIs 1485 -> 1263 us, astigmatic 1766
+// -> 1425.  (11x11, two blocks of 224 instead of three of 128, went from 1510 to
+// 1887 us for 800 000 ROIs: 14 warps instead of 12, but at 128 registers each.)
+__host__ __device__ constexpr int r1_scmos_threads(int box)
+{
+    return 2 * (128 * 4 * box * box + 1024) > 228 * 1024 ? 224 : 128;
+}
+
 template <int NCOLS>
 __device__ __forceinline__ void tmem_alloc(uint32_t *s_dst)  // one full warp
 {
@@ -1876,7 +1887,7 @@ __device__ __forceinline__ void fit_rois_r1(const KernelArgs &a, int64_t roi0, i
 // ROIs when held to 128 registers for a fourth block (with 52 bytes of
 // spills), 0.952 ms with its own 164 registers and three blocks.
 template <int MODEL, int BOX, bool SCMOS, bool TABLE, bool LM = false>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(SCMOS && !LM ? r1_scmos_threads(BOX) : 128)
     fit_kernel_r1(const KernelArgs a, const TileTable t)
 {
     extern __shared__ __align__(16) float smem[];
@@ -1885,9 +1896,13 @@ __global__ void __launch_bounds__(128)
     const int R = blockDim.x;
     uint32_t taddr = 0;
     if (SCMOS) {
-        if (threadIdx.x < 32) tmem_alloc<NCOLS>(&s_tmem);
+        if (threadIdx.x < 32) {
+            if (R > 128) tmem_alloc<2 * NCOLS>(&s_tmem);
+            else tmem_alloc<NCOLS>(&s_tmem);
+        }
         tmem_sync();
-        taddr = s_tmem + ((uint32_t)(((threadIdx.x >> 5) & 3) * 32) << 16);
+        taddr = s_tmem + (threadIdx.x >> 7) * NCOLS +
+                ((uint32_t)(((threadIdx.x >> 5) & 3) * 32) << 16);
     }
     if (!TABLE) {
         const int64_t roi0 = (int64_t)blockIdx.x * R;
@@ -1905,7 +1920,10 @@ __global__ void __launch_bounds__(128)
     }
     if (SCMOS) {
         tmem_sync();  // every warp's tensor-memory loads have completed
-        if (threadIdx.x < 32) tmem_dealloc<NCOLS>(s_tmem);
+        if (threadIdx.x < 32) {
+            if (R > 128) tmem_dealloc<2 * NCOLS>(s_tmem);
+            else tmem_dealloc<NCOLS>(s_tmem);
+        }
     }
 }
 

@@ -152,7 +152,7 @@ gmle_status init_mixed_set(gmle_ctx *ctx, MixedSet &m);
 void free_mixed_set(MixedSet &m);
 // ROIs per SM up to which a warp fits a ROI (alone, and of a submission whose
 // launches share the GPU), and from which one thread does (default_tuning).
-constexpr int kWarpLine = 16, kWarpTogether = 20, kPlainLine = 80,
+constexpr int kWarpLine = 20, kWarpTogether = 20, kPlainLine = 80,
               kPlainLineLarge = 64, kSubmissionLine = 200;
 // How a table launch picks its shape: from the context's tuning for the kind,
 // else the size-based default for a submission of `shape_rois` ROIs (0: this

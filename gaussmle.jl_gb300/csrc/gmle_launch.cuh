@@ -36,7 +36,8 @@ inline bool box_supported(int box) { return box_index(box) >= 0; }
 // The part of the odd boxes 5..15 (the most used sizes, with 8-lane kernels).
 __host__ __device__ constexpr bool main_box(int box) { return box >= 5 && box <= 15 && (box & 1); }
 
-// Largest block of the one-thread-per-ROI kernel (its __launch_bounds__).
+// Largest block of the one-thread-per-ROI kernel that can be asked for (the
+// default for large sCMOS batches may be r1_scmos_threads).
 constexpr int kMaxThreadsR1 = 128;
 
 // One launch of a model's kernel.  Plain (t.header == nullptr): ceil(a.n / rpb)
@@ -183,7 +184,8 @@ cudaError_t launch_one(const KernelArgs &a, const TileTable &t, const LaunchShap
     if (tpr != a.tpr) return cudaErrorInvalidValue;
     const int threads = rpb * tpr;
     const bool table = t.header != nullptr;
-    if (tpr == 1 && threads > kMaxThreadsR1) return cudaErrorInvalidConfiguration;
+    if (tpr == 1 && threads > (SCMOS && !shape.lm ? r1_scmos_threads(BOX) : kMaxThreadsR1))
+        return cudaErrorInvalidConfiguration;
     const size_t smem = launch_smem(MODEL, BOX, SCMOS, tpr, rpb, table);
     FitKernel kern;
     cudaError_t e = kernel_for<MODEL, BOX, SCMOS, PART>(tpr, table, shape.lm, &kern);
@@ -240,7 +242,8 @@ int table_blocks_one(int tpr, int rpb)
     // occupancy API answers one block per SM (it cannot know how many columns
     // a block takes).  Its residency is computed here from its registers,
     // shared memory and threads, and the 512 columns an SM holds.
-    return tmem_kernel_blocks_per_sm(kern, rpb * tpr, smem, tmem_var_cols(BOX));
+    return tmem_kernel_blocks_per_sm(kern, rpb * tpr, smem,
+                                     tmem_var_cols(BOX) * (rpb > 128 ? 2 : 1));
 }
 
 #define GMLE_CASE_PART0(CALL) CALL(5) CALL(7) CALL(9) CALL(11) CALL(13) CALL(15)

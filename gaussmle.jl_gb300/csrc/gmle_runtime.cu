@@ -99,12 +99,11 @@ namespace gmle_rt {
 // one thread): 12 000 ROIs 187 / 295, 25 000 246 / 294, 50 000 421 / 313.  That
 // line is drawn at 200 ROIs per SM.
 //
-// Up to 16 ROIs per SM (20 in a submission of several launches) a warp fits a
-// ROI: a pass is then a few hundred cycles instead of over a thousand, and all
-// warps are resident at once.  Measured (us, 4 lanes / 8 lanes / a warp): 200 ROIs
-// XYNB 11x11 45 / 43 / 23, astigmatic 15x15 99 / 72 / 37; 2 400 ROIs 45 / 43 / 31 and
-// 100 / 72 / 54 (4 lanes now: 37 and 68); 3 000 ROIs, in two waves of warps,
-// astigmatic 84.
+// Up to 20 ROIs per SM, its resident warps, a warp fits a ROI: a pass is then
+// shorter, and all warps run at once.  Measured (us, 4 lanes / a warp): 200 ROIs
+// XYNB 11x11 37 / 21; 3 000 ROIs XYNB 11x11 37 / 31, XYNBS 13x13 sCMOS 56 / 45,
+// astigmatic 15x15 67 / 56; 3 300 ROIs, a second wave of warps, 37 / 47, 56 / 67 and
+// 68 / 81.
 //
 // ROIs per block of the one-thread kernel: with sCMOS data 128, whose four warps
 // use their tensor-memory columns fully; Poisson data the block that lets
@@ -121,7 +120,7 @@ Tuning default_tuning(int num_sms, int box, bool scmos, int64_t n, int64_t toget
         return {32, gmle::warp_rois_per_block(num_sms, box, scmos, all)};
     if (all < (int64_t)line * num_sms) return {4, 32};
     const bool spread = together == 0 && n < (int64_t)256 * num_sms;
-    if (scmos) return {1, spread ? 96 : 128};
+    if (scmos) return {1, spread ? 96 : gmle::r1_scmos_threads(box)};
     if (spread) return {1, 32};
     int best = 64, most = 0;
     for (int rpb : {64, 128, 32}) {
@@ -144,7 +143,7 @@ Tuning pick_tuning(gmle_ctx *ctx, const gmle_fit_desc *d, int64_t n, int64_t tog
     auto it = ctx->tuning.find({d->model, d->box, (int)scmos});
     Tuning t = it != ctx->tuning.end() ? it->second
                                        : default_tuning(ctx->num_sms, d->box, scmos, n, together);
-    if (d->method == GMLE_METHOD_FISHER_LM && t.tpr != 1) {
+    if (d->method == GMLE_METHOD_FISHER_LM && (t.tpr != 1 || t.rois_per_block > 128)) {
         // the full-Hessian method runs one thread per ROI; 128-thread blocks
         // use the tensor memory of sCMOS variance tiles fully
         t.tpr = 1;

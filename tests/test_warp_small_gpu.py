@@ -1,6 +1,6 @@
 """Small batches of boxes 3..16, fitted with one warp per ROI by default: the edges
 of the lane grid (4, 8, 12, 15/16 pixels), blocks with empty warps, the table
-launch of a mixed submission, and both sides of the line of 16 ROIs per SM.
+launch of a mixed submission, and both sides of the line of 20 ROIs per SM.
 Compared with the oracle at the parity bar (test_boxes_gpu.check); the start
 point bit for bit (the sums run in the reference's order)."""
 import numpy as np
@@ -42,7 +42,7 @@ def test_start_point_is_the_references(ctx, model, camera, box):
     assert np.array_equal(prm, ref["params"])
 
 
-@pytest.mark.parametrize("n", [2431, 2432, 2433])
+@pytest.mark.parametrize("n", [3039, 3040, 3041])
 def test_both_sides_of_the_line(ctx, n):
     w = make_case("xynb-11-poisson", 0, 11, 0, n)
     params, crlb, llr, flags = run_gpu(ctx, w)
@@ -71,3 +71,22 @@ def test_table_launch_equals_plain(ctx):
         torch.cuda.synchronize()
         for a, b in zip(o, p):
             assert torch.equal(a.nan_to_num(7.0), b.nan_to_num(7.0)), w.name
+
+
+@pytest.mark.parametrize("model,camera,n", [(0, 2, 39_001), (3, 1, 39_137)])
+def test_blocks_of_seven_warps(ctx, model, camera, n):
+    """16x16 sCMOS batches from 256 ROIs per SM run in blocks of 224 ROIs, whose
+    fifth to seventh warps keep their variances in a second set of tensor-memory
+    columns: the same bits as in blocks of 128."""
+    w = make_case(f"m{model}-16-{camera}", model, 16, camera, 500)
+    rep = -(-n // w.n)
+    w.data = np.asfortranarray(np.tile(w.data, (1, 1, rep))[:, :, :n])
+    w.x_corners, w.y_corners = np.tile(w.x_corners, rep)[:n], np.tile(w.y_corners, rep)[:n]
+    got = run_gpu(ctx, w)
+    ctx.check(ctx.lib.gmle_set_tuning(ctx.handle, model, 16, camera, 1, 128))
+    try:
+        want = run_gpu(ctx, w)
+    finally:
+        ctx.check(ctx.lib.gmle_set_tuning(ctx.handle, model, 16, camera, 0, 0))
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b, equal_nan=True)
