@@ -137,8 +137,9 @@ gmle_status gmle_set_calibration(gmle_ctx *ctx, const float *variance, const flo
 /*
  * Synchronous fit of n ROIs from HOST memory into HOST memory: the whole GPU
  * branch of fit (src/interface.jl:220-262 and its ROIBatch twins).  Pinned
- * caller buffers are copied by DMA directly; pageable ones are staged through
- * the context's pinned buffers.  Transfers of one chunk overlap the fit of
+ * caller buffers are copied by DMA directly, and so are pageable ones where the
+ * GPU reads pageable memory; elsewhere these are staged through the context's
+ * pinned buffers.  Transfers of one chunk overlap the fit of
  * the previous one.  x_corners / y_corners may be NULL for Poisson fits;
  * flags may be NULL.
  */
@@ -275,9 +276,8 @@ typedef struct {
 /*
  * Fit a mixed batch (any mix of PSF models and box sizes 3..16) of
  * device-resident groups, enqueued on `stream` (used as given).  The groups of
- * each (camera family, model, box) present share one persistent,
- * work-stealing launch of that model's kernel; these launches run
- * concurrently.  A group of 65536 ROIs or more gets its own plain launch.  No
+ * each (camera family, model, box) present share one launch of that model's
+ * kernel, one block per tile of ROIs; these launches run concurrently.  A group of 65536 ROIs or more gets its own plain launch.  No
  * reference counterpart: the reference fits one (model, box) per fit() call
  * (src/interface.jl:177-291).
  */
