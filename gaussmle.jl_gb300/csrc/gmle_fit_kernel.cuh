@@ -174,6 +174,26 @@ __device__ __forceinline__ float half_erf(float t, float f)
     return copysignf(fmaf(-f, r * p, 0.5f), t);
 }
 
+// gauss_edge and half_erf of two edges in packed FP32
+__device__ __forceinline__ void half_erf2(float2 t, float2 &f, float2 &h)
+{
+    auto both = [](float x) { return make_float2(x, x); };
+    const float2 x = __fmul2_rn(__fmul2_rn(t, t), both(-0.72134752044448170368f));
+    f = make_float2(ex2_approx(x.x), ex2_approx(x.y));
+    const float2 q = __ffma2_rn(both(0.27577164466275354f), make_float2(fabsf(t.x), fabsf(t.y)),
+                                both(1.0f));
+    const float2 r = make_float2(rcp_approx(q.x), rcp_approx(q.y));
+    float2 p = both(0.5f * -0.22753699123859406f);
+    p = __ffma2_rn(p, r, both(0.5f * 0.8866637945175171f));
+    p = __ffma2_rn(p, r, both(0.5f * -0.6353994011878967f));
+    p = __ffma2_rn(p, r, both(0.5f * 0.6495586633682251f));
+    p = __ffma2_rn(p, r, both(0.5f * 0.09138870239257812f));
+    p = __ffma2_rn(p, r, both(0.5f * 0.2353251725435257f));
+    const float2 m = __fmul2_rn(r, p);
+    const float2 k = __ffma2_rn(make_float2(-f.x, -f.y), m, both(0.5f));
+    h = make_float2(copysignf(k.x, t.x), copysignf(k.y, t.y));
+}
+
 // ---- per-axis coefficients (hoisted out of the pixel loops) ----------------
 
 struct Axis {
@@ -224,7 +244,7 @@ __device__ __forceinline__ Axis make_axis(float c, float inv_s, float cst, float
 // time, took 31 per entry (43 with the width's); sharing them takes 21 (28).
 // With the Poisson terms' and Hessian terms' shorter forms: XYNB 11x11 Poisson,
 // 10^6 ROIs, 1909 -> 1644 us; XYNBS 13x13 sCMOS, 10^6, 3533 -> 3103; astigmatic
-// 15x15 Poisson, 300 000, 1436 -> 1207.
+// 15x15 Poisson, 300 000, 1436 -> 1207.  Row tables run it in pairs (edge_table).
 struct EdgeWalk {
     float pos;       // the last edge's position (t + 1/2)
     float h, f;      // erf / 2 and exp there
@@ -256,16 +276,13 @@ __device__ __forceinline__ EdgeWalk walk_start(int t0, const Axis &a)
     return w;
 }
 
-// The next pixel's entry: psf (integral_gaussian_1d, baselibrary.jl:8-14), its
-// derivatives d1, d2 by the position and z1, zq by the width's parameter, each
-// without the factor PSF of the other axis.
+// The entry between two neighbouring edges b and w: psf (integral_gaussian_1d,
+// baselibrary.jl:8-14), its derivatives d1, d2 by the position and z1, zq by the
+// width's parameter, each without the factor PSF of the other axis.
 template <bool SIG, bool SECOND>
-__device__ __forceinline__ void walk_entry(const Axis &a, EdgeWalk &w, float &psf, float &d1,
-                                           float &d2, float &z1, float &zq)
+__device__ __forceinline__ void edge_entry(const Axis &a, const EdgeWalk &b, const EdgeWalk &w,
+                                           float &psf, float &d1, float &d2, float &z1, float &zq)
 {
-    const EdgeWalk b = w;  // the lower edge
-    w.pos = b.pos + 1.0f;
-    walk_edge<SIG && SECOND>(a, w);
     // the true value is >= 0 (erf is increasing), so is the reference's; a
     // negative rounding residue of the tails is cut to 0
     psf = fmaxf(w.h - b.h, 0.0f);
@@ -275,6 +292,67 @@ __device__ __forceinline__ void walk_entry(const Axis &a, EdgeWalk &w, float &ps
     if (SIG) {
         z1 = a.kz * dg;
         if (SECOND) zq = fmaf(a.kq3, w.g3 - b.g3, a.kq * dg);
+    }
+}
+
+// The next pixel's entry of a walk (edge_entry).
+template <bool SIG, bool SECOND>
+__device__ __forceinline__ void walk_entry(const Axis &a, EdgeWalk &w, float &psf, float &d1,
+                                           float &d2, float &z1, float &zq)
+{
+    const EdgeWalk b = w;  // the lower edge
+    w.pos = b.pos + 1.0f;
+    walk_edge<SIG && SECOND>(a, w);
+    edge_entry<SIG, SECOND>(a, b, w, psf, d1, d2, z1, zq);
+}
+
+// walk_edge at two neighbouring edges in packed FP32: the same operations, so the
+// same bits, in 21 issued instructions (25 with the width's) instead of 34 (38).
+template <bool SIG>
+__device__ __forceinline__ void walk_edge2(const Axis &a, EdgeWalk &w0, EdgeWalk &w1)
+{
+    const float2 u = __fadd2_rn(make_float2(w0.pos, w1.pos), make_float2(-a.c, -a.c));
+    const float2 t = __fmul2_rn(u, make_float2(a.inv_s, a.inv_s));
+    float2 f, h;
+    half_erf2(t, f, h);
+    const float2 g = __fmul2_rn(u, f);
+    w0.f = f.x; w1.f = f.y;
+    w0.h = h.x; w1.h = h.y;
+    w0.g = g.x; w1.g = g.y;
+    if (SIG) {
+        const float2 g3 = __fmul2_rn(g, __fmul2_rn(u, u));
+        w0.g3 = g3.x; w1.g3 = g3.y;
+    }
+}
+
+// The entries of the R pixels from t0 on, their R + 1 edges in pairs: a row table
+// stands whole before the column loop, so its edges have no order to keep.  XYNB
+// 11x11 Poisson, 10^6 ROIs: 1631 -> 1622 us; XYNBS 13x13 sCMOS, 10^6: 3018 -> 2987;
+// astigmatic 15x15 Poisson, 300 000: 1192 -> 1181.
+template <bool SIG, int R>
+__device__ __forceinline__ void edge_table(const Axis &a, int t0, float *psf, float *d1, float *d2,
+                                           float *z1, float *zq)
+{
+    EdgeWalk w[R + 1];
+    const float first = (float)t0 - 0.5f;
+#pragma unroll
+    for (int e = 0; e <= R; e++) {
+        w[e].pos = first + (float)e;
+        w[e].g3 = 0.f;
+    }
+#pragma unroll
+    for (int e = 0; e <= R; e += 2) {
+        if (e < R) walk_edge2<SIG>(a, w[e], w[e + 1]);
+        else walk_edge<SIG>(a, w[e]);
+        float s1 = 0.f, s2 = 0.f;
+        if (e > 0) {
+            edge_entry<SIG, true>(a, w[e - 1], w[e], psf[e - 1], d1[e - 1], d2[e - 1], s1, s2);
+            if (SIG) { z1[e - 1] = s1; zq[e - 1] = s2; }
+        }
+        if (e < R) {
+            edge_entry<SIG, true>(a, w[e], w[e + 1], psf[e], d1[e], d2[e], s1, s2);
+            if (SIG) { z1[e] = s1; zq[e] = s2; }
+        }
     }
 }
 
@@ -1665,15 +1743,7 @@ __device__ __forceinline__ void fit_rois_r1(const KernelArgs &a, int64_t roi0, i
         const float N = th[S::IN], bg = th[S::IB];
         Axis ax, ay;
         make_axes<MODEL>(th, a, nk, ax, ay);
-        {
-            EdgeWalk wy = walk_start<SIG>(1, ay);
-#pragma unroll
-            for (int t = 0; t < BOX; t++) {
-                float s1 = 0.f, s2 = 0.f;
-                walk_entry<SIG, true>(ay, wy, py[t], yd1[t], yd2[t], s1, s2);
-                if (SIG) { ys1[t] = s1; ys2[t] = s2; }
-            }
-        }
+        edge_table<SIG, BOX>(ay, 1, py, yd1, yd2, ys1, ys2);
         EdgeWalk wx = walk_start<SIG>(1, ax);
         float xp, xd1, xd2, xs1 = 0.f, xs2 = 0.f;
         walk_entry<SIG, true>(ax, wx, xp, xd1, xd2, xs1, xs2);
@@ -2029,15 +2099,8 @@ __device__ __forceinline__ void fit_rois_tpr(const KernelArgs &a, int64_t roi0, 
         // this lane's share of its rows' table: row slots rx YR .. of the block
         // (slots past it are evaluated but not used)
         float ye[SIG ? 5 : 3][YR];
-        {
-            EdgeWalk wy = walk_start<SIG>(r0 + rx * YR + 1, ay);
-#pragma unroll
-            for (int t = 0; t < YR; t++) {
-                float z1 = 0.f, zq = 0.f;
-                walk_entry<SIG, true>(ay, wy, ye[0][t], ye[1][t], ye[2][t], z1, zq);
-                if constexpr (SIG) { ye[3][t] = z1; ye[4][t] = zq; }
-            }
-        }
+        edge_table<SIG, YR>(ay, r0 + rx * YR + 1, ye[0], ye[1], ye[2], ye[SIG ? 3 : 0],
+                            ye[SIG ? 4 : 0]);
         EdgeWalk wx = walk_start<SIG>(c0 + 1, ax);
         float xp, xd1, xd2, xs1 = 0.f, xs2 = 0.f;  // the lane's current column
         walk_entry<SIG, true>(ax, wx, xp, xd1, xd2, xs1, xs2);
