@@ -151,9 +151,9 @@ int nparams(int model);
 gmle_status init_mixed_set(gmle_ctx *ctx, MixedSet &m);
 void free_mixed_set(MixedSet &m);
 // ROIs per SM up to which a warp fits a ROI (alone, and of a submission whose
-// launches share the GPU), and from which one thread does (default_tuning).
-constexpr int kWarpLine = 20, kWarpTogether = 20, kPlainLine = 80,
-              kPlainLineLarge = 64, kSubmissionLine = 200;
+// launches share the GPU), and from which one thread does in such a submission
+// (default_tuning).
+constexpr int kWarpLine = 20, kWarpTogether = 20, kSubmissionLine = 200;
 // How a table launch picks its shape: from the context's tuning for the kind,
 // else the size-based default for a submission of `shape_rois` ROIs (0: this
 // one's); with request_rois > 0 by each group's own size instead, so that
@@ -192,7 +192,7 @@ gmle_status enqueue_table_launch(gmle_ctx *ctx, MixedSet &m, const TableLaunch &
 gmle_status enqueue_plan(gmle_ctx *ctx, MixedSet &m, const MixedPlan &plan, cudaStream_t s);
 gmle_status validate_groups(gmle_ctx *ctx, const gmle_group *groups, int32_t ngroups);
 Tuning pick_tuning(gmle_ctx *ctx, const gmle_fit_desc *d, int64_t n, int64_t together = 0);
-Tuning default_tuning(int num_sms, int box, bool scmos, int64_t n, int64_t together = 0);
+Tuning default_tuning(int num_sms, int model, int box, bool scmos, int64_t n, int64_t together = 0);
 gmle::KernelArgs make_args(gmle_ctx *ctx, const gmle_fit_desc *d, const float *data,
                            const int32_t *xc, const int32_t *yc, int64_t n, float *params,
                            float *crlb, float *llr, uint8_t *flags, int tpr);

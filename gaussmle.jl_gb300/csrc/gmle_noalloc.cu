@@ -225,7 +225,7 @@ extern "C" gmle_status gmle_fit_mixed_device_noalloc(const gmle_group *groups, i
         if (cnt == 0) continue;
         const gmle_fit_desc &d0 = groups[g_order[0]].desc;
         const bool scmos = d0.camera != GMLE_CAMERA_POISSON;
-        const gmle_rt::Tuning t = gmle_rt::default_tuning(S.num_sms, d0.box, scmos, together, together);
+        const gmle_rt::Tuning t = gmle_rt::default_tuning(S.num_sms, d0.model, d0.box, scmos, together, together);
         int64_t tiles = 0;
         for (int q = 0; q < cnt; q++) {
             const gmle_group &G = groups[g_order[q]];

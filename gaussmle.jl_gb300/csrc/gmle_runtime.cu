@@ -83,15 +83,32 @@ gmle_status check_desc(gmle_ctx *ctx, const gmle_fit_desc *d)
 
 namespace gmle_rt {
 
+// ROIs per SM up to which four lanes fit a ROI.  Both kernels' times are steps:
+// with four lanes a warp holds 8 ROIs, so 32, 64 and 96 ROIs per SM are one, two
+// and three warps per scheduler; with one thread per ROI it is one warp per
+// scheduler up to 128.  Measured with every model, box and camera family (us, four
+// lanes at 32 / 64 / 96 ROIs per SM, one thread up to 128): XYNB 11x11 37 / 45 / 53,
+// 60; 11x11 sCMOS 42 / 49 / 60, 64; XYNBS 9x9 41 / 49 / 60, 54; XYNBS 13x13 sCMOS
+// 56 / 70 / 88, 86; astigmatic 15x15 66 / 83 / 108, 105.  So the line is two warps per
+// scheduler; three where they still win, which takes a model with few sums (XYNB from
+// 8 pixels on; 9x9, split 5 + 4, does not: 48 and 46) or XYNBS 11x11 (64 and 70) and
+// 12x12 (74 and 87 with sCMOS; a few other boxes would gain up to 10 %); one for 3x3 and 5x5, which the lanes split most
+// unevenly (XYNBS 5x5 39 at 64, 35).  Of 16x16 sCMOS a third block does not fit the SM
+// (171 and 125), nor of the astigmatic 13x13 (134 and 92).
+static int plain_line(int model, int box, bool scmos)
+{
+    if (box == 3 || box == 5) return 32;
+    const bool three = model == GMLE_MODEL_XYNB
+                           ? box >= 8 && box != 9 && !(scmos && box == 16)
+                           : model == GMLE_MODEL_XYNBS && (box == 11 || box == 12);
+    return three ? 96 : 64;
+}
+
 // Launch shape when none is tuned, from the batch's size.
 //
 // One thread per ROI does the least work per ROI and wins as soon as the batch
 // gives every SM a few warps; several lanes per ROI shorten a fit's chain of
-// dependent passes when it does not.  Measured (us, 4 lanes / one thread):
-// 9 000 ROIs XYNB 11x11 45 / 60, 11x11 sCMOS 47 / 64, XYNBS 13x13 sCMOS 70 / 88,
-// astigmatic 15x15 sCMOS 92 / 130, 16x16 105 / 141; 12 000: 51 / 60, 57 / 64,
-// 90 / 88, 162 / 131, 205 / 145 (a second wave of blocks for the large boxes).  The
-// line is drawn at 80 ROIs per SM, from 15 pixels on at 64.
+// dependent passes when it does not (plain_line).
 //
 // `together` > 0: the launch is one of several, of `together` ROIs in all, that
 // share the SMs and are waited for together: the slowest launch's chain counts
@@ -111,15 +128,20 @@ namespace gmle_rt {
 // blocks of 128, two of which fit an SM, 1668 us in blocks of 64, three of
 // which fit).  Below 256 ROIs per SM smaller blocks spread over the SMs evenly
 // (20 000 XYNB 11x11 ROIs: 98 us in blocks of 32; 40 000 11x11 sCMOS: 131 us in
-// blocks of 96, 137 us of 128).
-Tuning default_tuning(int num_sms, int box, bool scmos, int64_t n, int64_t together)
+// blocks of 96, 137 us of 128).  Between 96 and 128 ROIs per SM one sCMOS block of
+// 128 per SM keeps a warp per scheduler, where blocks of 96 put a second block's on
+// some (19 400 ROIs, blocks of 96 / 128: XYNB 11x11 90 / 66 us, XYNBS 13x13 131 / 88,
+// astigmatic 15x15 178 / 129, XYNB 16x16 185 / 139).
+Tuning default_tuning(int num_sms, int model, int box, bool scmos, int64_t n, int64_t together)
 {
     const int64_t all = together > 0 ? together : n;
-    const int line = together > 0 ? kSubmissionLine : box >= 15 ? kPlainLineLarge : kPlainLine;
     if (all < (int64_t)(together > 0 ? kWarpTogether : kWarpLine) * num_sms)
         return {32, gmle::warp_rois_per_block(num_sms, box, scmos, all)};
-    if (all < (int64_t)line * num_sms) return {4, 32};
+    if (together > 0 ? all < (int64_t)kSubmissionLine * num_sms
+                     : n <= (int64_t)plain_line(model, box, scmos) * num_sms)
+        return {4, 32};
     const bool spread = together == 0 && n < (int64_t)256 * num_sms;
+    if (scmos && spread && n > (int64_t)96 * num_sms && n <= (int64_t)128 * num_sms) return {1, 128};
     if (scmos) return {1, spread ? 96 : gmle::r1_scmos_threads(box)};
     if (spread) return {1, 32};
     int best = 64, most = 0;
@@ -142,7 +164,7 @@ Tuning pick_tuning(gmle_ctx *ctx, const gmle_fit_desc *d, int64_t n, int64_t tog
     if (gmle::large_box(d->box)) return {32, gmle::warp_rois_per_block(ctx->num_sms, d->box, scmos, n)};
     auto it = ctx->tuning.find({d->model, d->box, (int)scmos});
     Tuning t = it != ctx->tuning.end() ? it->second
-                                       : default_tuning(ctx->num_sms, d->box, scmos, n, together);
+                                       : default_tuning(ctx->num_sms, d->model, d->box, scmos, n, together);
     if (d->method == GMLE_METHOD_FISHER_LM && (t.tpr != 1 || t.rois_per_block > 128)) {
         // the full-Hessian method runs one thread per ROI; 128-thread blocks
         // use the tensor memory of sCMOS variance tiles fully
@@ -548,7 +570,7 @@ gmle_status gmle_get_tuning(gmle_ctx *ctx, int32_t model, int32_t box, int32_t c
     const bool scmos = camera != GMLE_CAMERA_POISSON;
     auto it = ctx->tuning.find({model, box, (int)scmos});
     Tuning t = it != ctx->tuning.end() ? it->second
-                                       : default_tuning(ctx->num_sms, box, scmos, 1ll << 40);
+                                       : default_tuning(ctx->num_sms, model, box, scmos, 1ll << 40);
     *threads_per_roi = t.tpr;
     *rois_per_block = t.rois_per_block;
     return GMLE_OK;

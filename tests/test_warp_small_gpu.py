@@ -49,6 +49,29 @@ def test_both_sides_of_the_line(ctx, n):
     check(w, params, crlb, flags)
 
 
+@pytest.mark.parametrize("model,box,camera,n", [(1, 5, 0, 4864), (1, 5, 0, 4865),
+                                                (1, 9, 0, 9728), (1, 9, 0, 9729),
+                                                (0, 11, 2, 14592), (0, 11, 2, 14593),
+                                                (0, 11, 2, 19456), (0, 11, 2, 19457)])
+def test_both_sides_of_the_one_thread_lines(ctx, model, box, camera, n):
+    """32, 64 and 96 ROIs per SM, where one thread per ROI takes over, and 128, where
+    its sCMOS blocks go from 128 ROIs to 96 (152 SMs): the bits of the shape set
+    explicitly, and the oracle's results at the parity bar."""
+    w = make_case(f"m{model}-{box}-{camera}", model, box, camera, n)
+    got = run_gpu(ctx, w)
+    line = 32 if box == 5 else 64 if box == 9 else 96
+    shape = (4, 32) if n <= line * 152 else (1, 32 if not camera else 128 if n <= 128 * 152 else 96)
+    ctx.check(ctx.lib.gmle_set_tuning(ctx.handle, model, box, camera, *shape))
+    try:
+        want = run_gpu(ctx, w)
+    finally:
+        ctx.check(ctx.lib.gmle_set_tuning(ctx.handle, model, box, camera, 0, 0))
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b, equal_nan=True)
+    if box > 5:
+        check(w, got[0], got[1], got[3])
+
+
 def test_table_launch_equals_plain(ctx):
     """A mixed submission below its line: the same warps, from a table."""
     torch = pytest.importorskip("torch")
