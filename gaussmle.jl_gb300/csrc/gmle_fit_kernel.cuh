@@ -154,34 +154,32 @@ __device__ __forceinline__ float gauss_edge(float t)
 {
     return ex2_approx(__fmul_rn(t, t) * -0.72134752044448170368f);
 }
-// erf(t / sqrt 2) / 2, given f = exp(-t^2 / 2) (the caller's gauss_edge at the
-// same edge).  Hastings' form (Abramowitz & Stegun 7.1.26): erf(x) = 1 - e r P(r)
-// for x >= 0, e = exp(-x^2), r = 1 / (1 + p x), here with P of degree 5 refitted
-// by a least-squares (Lawson) minimax fit of exp(-x^2) erfcx(x) on [0, 6]: p =
-// 0.39, 8.3e-9 largest error in exact arithmetic, below 4.5e-7 absolute (of erf)
-// evaluated in FP32 (most of it near x = 0, from 1 - e r P(r)); erf(-x) =
-// -erf(x).  The factor 1/2 is in P's coefficients, 1/sqrt 2 in p.  Checked against
-// the library's erff by tests/test_math_gpu.py.
-__device__ __forceinline__ float half_erf(float t, float f)
+// erf(x) / 2, given e = exp(-x^2) (the caller's gauss_edge at the same edge).
+// Hastings' form (Abramowitz & Stegun 7.1.26): erf(x) = 1 - e r P(r) for x >= 0,
+// r = 1 / (1 + p x), here with P of degree 5 refitted by a least-squares
+// (Lawson) minimax fit of exp(-x^2) erfcx(x) on [0, 6]: p = 0.39, 8.3e-9 largest
+// error in exact arithmetic, 4.3e-7 absolute (of erf) evaluated in FP32 (most of
+// it near x = 0, from 1 - e r P(r)); erf(-x) = -erf(x).  The factor 1/2 is in P's
+// coefficients.  Checked against the library's erff by tests/test_math_gpu.py.
+__device__ __forceinline__ float half_erf(float x, float e)
 {
-    const float r = rcp_approx(fmaf(0.27577164466275354f, fabsf(t), 1.0f));
+    const float r = rcp_approx(fmaf(0.39f, fabsf(x), 1.0f));
     float p = 0.5f * -0.22753699123859406f;
     p = fmaf(p, r, 0.5f * 0.8866637945175171f);
     p = fmaf(p, r, 0.5f * -0.6353994011878967f);
     p = fmaf(p, r, 0.5f * 0.6495586633682251f);
     p = fmaf(p, r, 0.5f * 0.09138870239257812f);
     p = fmaf(p, r, 0.5f * 0.2353251725435257f);
-    return copysignf(fmaf(-f, r * p, 0.5f), t);
+    return copysignf(fmaf(-e, r * p, 0.5f), x);
 }
 
-// gauss_edge and half_erf of two edges in packed FP32
-__device__ __forceinline__ void half_erf2(float2 t, float2 &f, float2 &h)
+// gauss_edge (at t) and half_erf (at x) of two edges in packed FP32
+__device__ __forceinline__ void half_erf2(float2 t, float2 x, float2 &f, float2 &h)
 {
-    auto both = [](float x) { return make_float2(x, x); };
-    const float2 x = __fmul2_rn(__fmul2_rn(t, t), both(-0.72134752044448170368f));
-    f = make_float2(ex2_approx(x.x), ex2_approx(x.y));
-    const float2 q = __ffma2_rn(both(0.27577164466275354f), make_float2(fabsf(t.x), fabsf(t.y)),
-                                both(1.0f));
+    auto both = [](float v) { return make_float2(v, v); };
+    const float2 y = __fmul2_rn(__fmul2_rn(t, t), both(-0.72134752044448170368f));
+    f = make_float2(ex2_approx(y.x), ex2_approx(y.y));
+    const float2 q = __ffma2_rn(both(0.39f), make_float2(fabsf(x.x), fabsf(x.y)), both(1.0f));
     const float2 r = make_float2(rcp_approx(q.x), rcp_approx(q.y));
     float2 p = both(0.5f * -0.22753699123859406f);
     p = __ffma2_rn(p, r, both(0.5f * 0.8866637945175171f));
@@ -191,7 +189,7 @@ __device__ __forceinline__ void half_erf2(float2 t, float2 &f, float2 &h)
     p = __ffma2_rn(p, r, both(0.5f * 0.2353251725435257f));
     const float2 m = __fmul2_rn(r, p);
     const float2 k = __ffma2_rn(make_float2(-f.x, -f.y), m, both(0.5f));
-    h = make_float2(copysignf(k.x, t.x), copysignf(k.y, t.y));
+    h = make_float2(copysignf(k.x, x.x), copysignf(k.y, x.y));
 }
 
 // ---- per-axis coefficients (hoisted out of the pixel loops) ----------------
@@ -199,6 +197,7 @@ __device__ __forceinline__ void half_erf2(float2 t, float2 &f, float2 &h)
 struct Axis {
     float c;           // centre (x or y, ROI pixels)
     float inv_s;       // 1 / sigma (pixels)
+    float sq;          // sqrt(1/2 / s^2): integral_gaussian_1d, baselibrary.jl:8-14
     float cst;         // -N / (sqrt(2 pi) s): derivative_integral_gaussian_1d, baselibrary.jl:21-33
     float cst2;        // cst / s^2
     // derivatives by the width's parameter (s itself, or z): baselibrary.jl:40-52
@@ -216,6 +215,7 @@ __device__ __forceinline__ Axis make_axis(float c, float inv_s, float cst, float
     Axis a;
     a.c = c;
     a.inv_s = inv_s;
+    a.sq = 0.70710678118654752f * inv_s;
     a.cst = cst;
     const float is2 = inv_s * inv_s;
     a.cst2 = cst * is2;
@@ -241,10 +241,15 @@ __device__ __forceinline__ Axis make_axis(float c, float inv_s, float cst, float
 // bound by issue and fixed-latency waits (issue slots 58-66 % busy, FMA pipe
 // 53-59 %), and the tables were a quarter of their instructions: both edges'
 // products per pixel, with the reference's two roundings of u told apart at run
-// time, took 31 per entry (43 with the width's); sharing them takes 21 (28).
-// With the Poisson terms' and Hessian terms' shorter forms: XYNB 11x11 Poisson,
-// 10^6 ROIs, 1909 -> 1644 us; XYNBS 13x13 sCMOS, 10^6, 3533 -> 3103; astigmatic
-// 15x15 Poisson, 300 000, 1436 -> 1207.  Row tables run it in pairs (edge_table).
+// time, took 31 per entry (43 with the width's); sharing them takes 22 (29).
+// With the Hessian terms' FMA chains and row tables in pairs (edge_table): XYNB 11x11
+// Poisson, 10^6 ROIs, 1909 -> 1669 us; XYNBS 13x13 sCMOS, 10^6, 3533 -> 2992 (two
+// columns per trip included); astigmatic 15x15 Poisson, 300 000, 1436 -> 1241.
+// erf's argument is u sqrt(1/2 / s^2), rounded, as the reference forms it: with 1/sqrt 2
+// taken into the polynomial's p the same entries cost 1 % less (XYNB 1622 us, with
+// the shorter Poisson terms that likelihood_terms names) and are as exact, but every mu of
+// a Poisson fit then has another last bit, and its p-values another error
+// (final_pixel): 2.0e-5 of their norm for 7x7 boxes, 2.8e-5 for astigmatic 13x13.
 struct EdgeWalk {
     float pos;       // the last edge's position (t + 1/2)
     float h, f;      // erf / 2 and exp there
@@ -257,7 +262,7 @@ __device__ __forceinline__ void walk_edge(const Axis &a, EdgeWalk &w)
     const float u = w.pos - a.c;
     const float t = u * a.inv_s;
     w.f = gauss_edge(t);
-    w.h = half_erf(t, w.f);
+    w.h = half_erf(__fmul_rn(u, a.sq), w.f);
     // (rounded products: which of an entry's differences the compiler would
     // contract into FMAs could differ between the plain and the table kernels,
     // whose results are the same bits)
@@ -307,14 +312,14 @@ __device__ __forceinline__ void walk_entry(const Axis &a, EdgeWalk &w, float &ps
 }
 
 // walk_edge at two neighbouring edges in packed FP32: the same operations, so the
-// same bits, in 21 issued instructions (25 with the width's) instead of 34 (38).
+// same bits, in 22 issued instructions (26 with the width's) instead of 36 (40).
 template <bool SIG>
 __device__ __forceinline__ void walk_edge2(const Axis &a, EdgeWalk &w0, EdgeWalk &w1)
 {
     const float2 u = __fadd2_rn(make_float2(w0.pos, w1.pos), make_float2(-a.c, -a.c));
     const float2 t = __fmul2_rn(u, make_float2(a.inv_s, a.inv_s));
     float2 f, h;
-    half_erf2(t, f, h);
+    half_erf2(t, __fmul2_rn(u, make_float2(a.sq, a.sq)), f, h);
     const float2 g = __fmul2_rn(u, f);
     w0.f = f.x; w1.f = f.y;
     w0.h = h.x; w1.h = h.y;
@@ -1240,16 +1245,19 @@ template <int MODEL> struct Slots {
 
 // Likelihood terms of one pixel: compute_likelihood_terms, Poisson
 // src/camera_models.jl:19-34 and sCMOS :36-42 (1/x by rcp_approx, 1 ulp).
-// Poisson: d / mu - 1 with one rounding, and d / mu^2 = (cf + 1) / mu from it.
+// Poisson: q = d / mu is rounded before both cf = q - 1 and df = q / mu.  df from cf
+// (cf / mu + 1 / mu) saves an operation, but of a pixel with d << mu it is then only
+// good to 2^-24 / mu; and a cf rounded once moves N and bg by an ulp in 30 % of the
+// fits, and with them the rounding of the log-likelihood ratio (final_pixel).
 template <bool SCMOS>
 __device__ __forceinline__ void likelihood_terms(float d, float v, float mu, float &cf, float &df)
 {
     if (!SCMOS) {
         const float rm = rcp_approx(mu);
-        const float c = fmaf(d, rm, -1.0f);
+        const float q = __fmul_rn(d, rm);
         const bool pos = mu > 0.01f;
-        cf = pos ? fminf(c, 1e4f) : 0.f;
-        df = pos ? fminf(fmaf(c, rm, rm), 1e4f) : 0.f;
+        cf = pos ? fminf(__fadd_rn(q, -1.0f), 1e4f) : 0.f;
+        df = pos ? fminf(__fmul_rn(q, rm), 1e4f) : 0.f;
     } else {
         const float rv = rcp_approx(mu + v);
         cf = (d - mu) * rv;
@@ -1262,8 +1270,9 @@ __device__ __forceinline__ void likelihood_terms(float d, float v, float mu, flo
 __device__ __forceinline__ void likelihood_terms_uncapped(float d, float mu, float &cf, float &df)
 {
     const float rm = rcp_approx(mu);
-    cf = fmaf(d, rm, -1.0f);
-    df = fmaf(cf, rm, rm);
+    const float q = __fmul_rn(d, rm);
+    cf = __fadd_rn(q, -1.0f);
+    df = __fmul_rn(q, rm);
 }
 
 // Whether a Poisson fit's pixel terms need no mu > 0.01 test and no 1e4 cap
@@ -1281,8 +1290,9 @@ __device__ __forceinline__ bool uncapped(float N, float bg, float dmax)
 // sm_100's add/mul/fma .f32x2 take one issue slot for two FP32 operations, each
 // half rounded exactly like the scalar operation.  The one-thread kernel's
 // Newton pixel loop runs rows (t, t+1) of a column as one pair.  Each half
-// evaluates likelihood_terms / _uncapped's expressions (d - mu as
-// fma(mu, -1, d): one rounding, like the subtraction).
+// evaluates likelihood_terms / _uncapped's expressions with every operation
+// rounded as written, none contracted into an FMA (d - mu as fma(mu, -1, d):
+// one rounding, like the subtraction).
 __device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
 
 template <bool SCMOS, bool UNCAPPED>
@@ -1296,8 +1306,9 @@ __device__ __forceinline__ void likelihood_terms2(float2 d, float2 v, float2 mu,
         df = rv;
     } else {
         const float2 rm = make_float2(rcp_approx(mu.x), rcp_approx(mu.y));
-        const float2 c = __ffma2_rn(d, rm, f2(-1.0f));
-        const float2 e = __ffma2_rn(c, rm, rm);
+        const float2 q = __fmul2_rn(d, rm);
+        const float2 c = __fadd2_rn(q, f2(-1.0f));
+        const float2 e = __fmul2_rn(q, rm);
         if constexpr (UNCAPPED) {
             cf = c;
             df = e;
@@ -1388,6 +1399,8 @@ __device__ __forceinline__ float qsym(const float (&Q)[NB][NB], int p, int q)
 // Per pixel of the final pass: the LLR term (compute_log_likelihood,
 // src/camera_models.jl:60-96) and the Fisher weight sums Q_pq += b_p b_q w,
 // w = 1/variance over pixels with mu > 0 (src/unified_kernel.jl:378-396).
+// A Poisson ratio's terms, d ln d in size, cancel: it is off by some 1e-4, and the last
+// bit of mu decides by which (p-values of 7x7 boxes: 2.7e-5 of their norm).
 // FAST_LOG: the Poisson LLR's logarithms by log_approx (the final pass, whose
 // LLR is an output only); the full-Hessian passes, which accept or reject a
 // step on the LLR, keep the library's logf.

@@ -20,10 +20,9 @@ __global__ void math_selftest_kernel(const float *__restrict__ x, int64_t n, flo
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float v = x[i];
-    // the fit's erf takes the edge offset over sigma (here sqrt(2) v) and the
-    // exponential of the same edge
-    const float t = v * 1.41421356237309515f;
-    out[i] = 2.0f * gmle::half_erf(t, gmle::gauss_edge(t));
+    // the fit's erf takes exp(-v^2) from gauss_edge at the same edge, whose
+    // argument is the edge offset over sigma (here sqrt(2) v)
+    out[i] = 2.0f * gmle::half_erf(v, gmle::gauss_edge(v * 1.41421356237309515f));
     out[n + i] = erff(v);
     out[2 * n + i] = gmle::gauss_edge(v);
     out[3 * n + i] = expf(-0.5f * (v * v));
