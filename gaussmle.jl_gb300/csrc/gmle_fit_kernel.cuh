@@ -32,6 +32,8 @@
 
 #include <type_traits>
 
+#include "gmle_corners.h"
+
 namespace gmle {
 
 struct KernelArgs {
@@ -1024,7 +1026,7 @@ __device__ __forceinline__ bool stage_r1(const KernelArgs &a, float *spix, int64
         long long base = 0;
         if (ok) {
             const int32_t x0 = a.xc[roi0 + g], y0 = a.yc[roi0 + g];
-            ok = x0 >= 1 && y0 >= 1 && x0 + BOX - 1 <= a.nx && y0 + BOX - 1 <= a.ny;
+            ok = corner_inside(x0, y0, BOX, a.ny, a.nx);
             if (!ok) atomicAdd(a.bad_corners, 1ull);
             base = ok ? (long long)(y0 - 1) + (long long)a.ny * (long long)(x0 - 1) : 0;
         }
@@ -1105,7 +1107,7 @@ __device__ __forceinline__ bool stage_r1(const KernelArgs &a, float *spix, int64
         long long base = 0;
         if (ok) {
             const int32_t x0 = a.xc[roi0 + r0 + l], y0 = a.yc[roi0 + r0 + l];
-            ok = x0 >= 1 && y0 >= 1 && x0 + BOX - 1 <= a.nx && y0 + BOX - 1 <= a.ny;
+            ok = corner_inside(x0, y0, BOX, a.ny, a.nx);
             if (!ok) atomicAdd(a.bad_corners, 1ull);
             base = ok ? (long long)(y0 - 1) + (long long)a.ny * (long long)(x0 - 1) : 0;
         }
@@ -1211,7 +1213,7 @@ __device__ __forceinline__ void stage_block(const KernelArgs &a, float *spix, fl
         long long base = 0;
         if (SCMOS && ok) {
             const int32_t x0 = a.xc[roi0 + g], y0 = a.yc[roi0 + g];
-            ok = x0 >= 1 && y0 >= 1 && x0 + BOX - 1 <= a.nx && y0 + BOX - 1 <= a.ny;
+            ok = corner_inside(x0, y0, BOX, a.ny, a.nx);
             if (!ok) atomicAdd(a.bad_corners, 1ull);
             base = (long long)(y0 - 1) + (long long)a.ny * (long long)(x0 - 1);
         }

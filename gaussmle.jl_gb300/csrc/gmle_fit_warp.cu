@@ -320,7 +320,7 @@ __device__ __forceinline__ void fit_roi_warp(const KernelArgs &a, const int box,
     long long base = 0;
     if (SCMOS) {
         const int32_t x0 = a.xc[roi], y0 = a.yc[roi];
-        ok = x0 >= 1 && y0 >= 1 && x0 + box - 1 <= a.nx && y0 + box - 1 <= a.ny;
+        ok = corner_inside(x0, y0, box, a.ny, a.nx);
         if (!ok && lane == 0) atomicAdd(a.bad_corners, 1ull);
         base = ok ? (long long)(y0 - 1) + (long long)a.ny * (x0 - 1) : 0;
     }

@@ -53,6 +53,7 @@ def nvcc() -> str:
 
 def _deps() -> list[Path]:
     return sorted(CSRC.glob("*.cu")) + sorted(CSRC.glob("*.cuh")) + \
+        sorted(CSRC.glob("*.h")) + \
         sorted((REPO_ROOT / "include").glob("*.h")) + [Path(__file__)]
 
 
