@@ -310,6 +310,14 @@ gmle_status flush_slot(gmle_ctx *ctx, Slot &s)
     return GMLE_OK;
 }
 
+// After a failed call: nothing queued may still read or write the caller's memory, nor
+// may a slot's finished chunk be copied to it by the next call.
+void abandon_fit(gmle_ctx *ctx)
+{
+    for (cudaStream_t s : {ctx->s_h2d, ctx->s_fit, ctx->s_d2h}) cudaStreamSynchronize(s);
+    for (Slot &s : ctx->slots) s.pending = false;
+}
+
 gmle_status check_corners_host(gmle_ctx *ctx, const gmle_fit_desc *d, const int32_t *xc,
                                const int32_t *yc, int64_t n)
 {
@@ -501,65 +509,70 @@ gmle_status gmle_fit(gmle_ctx *ctx, const gmle_fit_desc *desc, const float *data
         st = ensure_slot(ctx, s, chunk, b2, !(in_pinned && out_pinned));
         if (st != GMLE_OK) return st;
     }
-    int k = 0;
-    for (int64_t off = 0; off < n; off += chunk, k ^= 1) {
-        Slot &s = ctx->slots[k];
-        const int64_t m = std::min(chunk, n - off);
-        // The slot's previous chunk must be out before its buffers are reused.
-        st = flush_slot(ctx, s);
-        if (st != GMLE_OK) return st;
-        CK(cudaStreamWaitEvent(ctx->s_h2d, s.d2h_done, 0), "cudaStreamWaitEvent");
-        const float *src = data + off * b2;
-        if (!in_pinned) {
-            CK(cudaEventSynchronize(s.h2d_done), "cudaEventSynchronize");
-            std::memcpy(s.h_data, src, sizeof(float) * m * b2);
-            src = s.h_data;
+    auto run = [&]() -> gmle_status {
+        int k = 0;
+        for (int64_t off = 0; off < n; off += chunk, k ^= 1) {
+            Slot &s = ctx->slots[k];
+            const int64_t m = std::min(chunk, n - off);
+            // The slot's previous chunk must be out before its buffers are reused.
+            const gmle_status st = flush_slot(ctx, s);
+            if (st != GMLE_OK) return st;
+            CK(cudaStreamWaitEvent(ctx->s_h2d, s.d2h_done, 0), "cudaStreamWaitEvent");
+            const float *src = data + off * b2;
+            if (!in_pinned) {
+                CK(cudaEventSynchronize(s.h2d_done), "cudaEventSynchronize");
+                std::memcpy(s.h_data, src, sizeof(float) * m * b2);
+                src = s.h_data;
+            }
+            CK(cudaMemcpyAsync(s.data, src, sizeof(float) * m * b2, cudaMemcpyHostToDevice, ctx->s_h2d),
+               "H2D data");
+            if (scmos) {
+                CK(cudaMemcpyAsync(s.xc, x_corners + off, sizeof(int32_t) * m, cudaMemcpyHostToDevice,
+                                   ctx->s_h2d), "H2D corners");
+                CK(cudaMemcpyAsync(s.yc, y_corners + off, sizeof(int32_t) * m, cudaMemcpyHostToDevice,
+                                   ctx->s_h2d), "H2D corners");
+            }
+            CK(cudaEventRecord(s.h2d_done, ctx->s_h2d), "cudaEventRecord");
+            CK(cudaStreamWaitEvent(ctx->s_fit, s.h2d_done, 0), "cudaStreamWaitEvent");
+            KernelArgs a = make_args(ctx, desc, s.data, scmos ? s.xc : nullptr, scmos ? s.yc : nullptr,
+                                     m, s.params, s.crlb, s.llr, s.flags, t.tpr);
+            CK(launch(ctx, desc, a, t.rois_per_block, ctx->s_fit), "fit kernel launch");
+            CK(cudaEventRecord(s.fit_done, ctx->s_fit), "cudaEventRecord");
+            CK(cudaStreamWaitEvent(ctx->s_d2h, s.fit_done, 0), "cudaStreamWaitEvent");
+            float *op = out_pinned ? params + off * P : s.h_params;
+            float *oc = out_pinned ? crlb + off * P : s.h_crlb;
+            float *ol = out_pinned ? llr + off : s.h_llr;
+            uint8_t *of = out_pinned ? (flags ? flags + off : nullptr) : s.h_flags;
+            CK(cudaMemcpyAsync(op, s.params, sizeof(float) * m * P, cudaMemcpyDeviceToHost, ctx->s_d2h),
+               "D2H params");
+            CK(cudaMemcpyAsync(oc, s.crlb, sizeof(float) * m * P, cudaMemcpyDeviceToHost, ctx->s_d2h),
+               "D2H crlb");
+            CK(cudaMemcpyAsync(ol, s.llr, sizeof(float) * m, cudaMemcpyDeviceToHost, ctx->s_d2h),
+               "D2H llr");
+            if (of)
+                CK(cudaMemcpyAsync(of, s.flags, m, cudaMemcpyDeviceToHost, ctx->s_d2h), "D2H flags");
+            CK(cudaEventRecord(s.d2h_done, ctx->s_d2h), "cudaEventRecord");
+            if (!out_pinned) {
+                s.pending = true;
+                s.dst_params = params + off * P;
+                s.dst_crlb = crlb + off * P;
+                s.dst_llr = llr + off;
+                s.dst_flags = flags ? flags + off : nullptr;
+                s.pend_rois = m;
+                s.pend_p = P;
+            }
         }
-        CK(cudaMemcpyAsync(s.data, src, sizeof(float) * m * b2, cudaMemcpyHostToDevice, ctx->s_h2d),
-           "H2D data");
-        if (scmos) {
-            CK(cudaMemcpyAsync(s.xc, x_corners + off, sizeof(int32_t) * m, cudaMemcpyHostToDevice,
-                               ctx->s_h2d), "H2D corners");
-            CK(cudaMemcpyAsync(s.yc, y_corners + off, sizeof(int32_t) * m, cudaMemcpyHostToDevice,
-                               ctx->s_h2d), "H2D corners");
+        for (Slot &s : ctx->slots) {
+            const gmle_status st = flush_slot(ctx, s);
+            if (st != GMLE_OK) return st;
         }
-        CK(cudaEventRecord(s.h2d_done, ctx->s_h2d), "cudaEventRecord");
-        CK(cudaStreamWaitEvent(ctx->s_fit, s.h2d_done, 0), "cudaStreamWaitEvent");
-        KernelArgs a = make_args(ctx, desc, s.data, scmos ? s.xc : nullptr, scmos ? s.yc : nullptr,
-                                 m, s.params, s.crlb, s.llr, s.flags, t.tpr);
-        CK(launch(ctx, desc, a, t.rois_per_block, ctx->s_fit), "fit kernel launch");
-        CK(cudaEventRecord(s.fit_done, ctx->s_fit), "cudaEventRecord");
-        CK(cudaStreamWaitEvent(ctx->s_d2h, s.fit_done, 0), "cudaStreamWaitEvent");
-        float *op = out_pinned ? params + off * P : s.h_params;
-        float *oc = out_pinned ? crlb + off * P : s.h_crlb;
-        float *ol = out_pinned ? llr + off : s.h_llr;
-        uint8_t *of = out_pinned ? (flags ? flags + off : nullptr) : s.h_flags;
-        CK(cudaMemcpyAsync(op, s.params, sizeof(float) * m * P, cudaMemcpyDeviceToHost, ctx->s_d2h),
-           "D2H params");
-        CK(cudaMemcpyAsync(oc, s.crlb, sizeof(float) * m * P, cudaMemcpyDeviceToHost, ctx->s_d2h),
-           "D2H crlb");
-        CK(cudaMemcpyAsync(ol, s.llr, sizeof(float) * m, cudaMemcpyDeviceToHost, ctx->s_d2h),
-           "D2H llr");
-        if (of)
-            CK(cudaMemcpyAsync(of, s.flags, m, cudaMemcpyDeviceToHost, ctx->s_d2h), "D2H flags");
-        CK(cudaEventRecord(s.d2h_done, ctx->s_d2h), "cudaEventRecord");
-        if (!out_pinned) {
-            s.pending = true;
-            s.dst_params = params + off * P;
-            s.dst_crlb = crlb + off * P;
-            s.dst_llr = llr + off;
-            s.dst_flags = flags ? flags + off : nullptr;
-            s.pend_rois = m;
-            s.pend_p = P;
-        }
-    }
-    for (Slot &s : ctx->slots) {
-        st = flush_slot(ctx, s);
-        if (st != GMLE_OK) return st;
-    }
-    CK(cudaStreamSynchronize(ctx->s_d2h), "cudaStreamSynchronize");
-    CK(cudaStreamSynchronize(ctx->s_fit), "cudaStreamSynchronize");
-    return GMLE_OK;
+        CK(cudaStreamSynchronize(ctx->s_d2h), "cudaStreamSynchronize");
+        CK(cudaStreamSynchronize(ctx->s_fit), "cudaStreamSynchronize");
+        return GMLE_OK;
+    };
+    st = run();
+    if (st != GMLE_OK) abandon_fit(ctx);
+    return st;
 }
 
 gmle_status gmle_get_tuning(gmle_ctx *ctx, int32_t model, int32_t box, int32_t camera,

@@ -1,0 +1,96 @@
+"""The library's host code without a GPU: its objects linked with a fake CUDA runtime
+(fake/fake_cuda.cpp) that logs the calls, keeps device memory on the host and fails
+a named call.  Kernels do nothing there: only what the host does is tested."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import ROOT
+from gaussmle_gb300 import build
+from gaussmle_gb300.constraints import default_constraints
+from gaussmle_gb300.fitter import make_desc
+from gaussmle_gb300.models import GaussianXYNB
+
+SMS = 152
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    build.build(force=not build.BUILD_DIR.exists())
+    out = tmp_path_factory.mktemp("fake") / "libfake.so"
+    objs = [str(build.BUILD_DIR / (u[1] + ".o")) for u in build.UNITS]
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(build.nvcc()))), "include")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", f"-I{cuda}", "-o", str(out),
+                    str(ROOT / "tests" / "fake" / "fake_cuda.cpp"), *objs, "-Wl,-Bsymbolic",
+                    "-lpthread"], check=True)
+    lib = C.CDLL(str(out))
+    lib.fake_log.restype = C.c_char_p
+    lib.gmle_last_error.restype = C.c_char_p
+    yield lib
+    out.unlink()
+
+
+@pytest.fixture
+def ctx(lib):
+    lib.fake_host_pages(0)
+    lib.fake_fail(b"", 0)
+    c = C.c_void_p()
+    assert lib.gmle_create(C.byref(c), 0) == 0
+    yield c
+    lib.fake_fail(b"", 0)
+    lib.gmle_destroy(c)
+
+
+def calls(lib, name):
+    """(stream, *numbers) of every logged call of `name`."""
+    rows = (r.split() for r in lib.fake_log().decode().splitlines())
+    return [tuple(int(v) for v in r[1:]) for r in rows if r[0] == name]
+
+
+def p(a):
+    return a.ctypes.data_as(C.c_void_p) if a is not None else None
+
+
+BOX = 3
+CHUNK = (64 << 20) // (4 * BOX * BOX)  # gmle_fit's chunk, 64 MiB of pixels
+
+
+def desc(box=BOX):
+    psf = GaussianXYNB(1.3)
+    return make_desc(psf, box, 20, default_constraints(psf, box), 0)
+
+
+def host_fit(lib, ctx, data, n, fill=7.0):
+    out = [np.full((n, 4), fill, np.float32), np.full((n, 4), fill, np.float32),
+           np.full(n, fill, np.float32), np.full(n, int(fill), np.uint8)]
+    return lib.gmle_fit(ctx, C.byref(desc()), p(data), None, None, C.c_int64(n),
+                        *map(p, out)), out
+
+
+@pytest.mark.parametrize("host_pages", [0, 1])
+@pytest.mark.parametrize("name,nth", [("cudaMemcpyAsync", 6), ("launch", 3), ("cudaEventRecord", 9)])
+def test_a_failed_fit_leaves_nothing_behind(lib, ctx, host_pages, name, nth):
+    """Three chunks, an error in the second or third: every stream has run dry before
+    the call returns, and the next call writes to its own buffers only."""
+    lib.gmle_destroy(ctx)
+    lib.fake_host_pages(host_pages)
+    assert lib.gmle_create(C.byref(ctx), 0) == 0
+    data = np.zeros((2 * CHUNK + 10, BOX * BOX), np.float32)
+    lib.fake_clear()
+    lib.fake_fail(name.encode(), nth)
+    st, out = host_fit(lib, ctx, data, len(data))
+    assert st != 0 and b"fake error" in lib.gmle_last_error(ctx)
+    log = lib.fake_log().decode().splitlines()
+    used = {r.split()[1] for r in log if r.startswith(("cudaMemcpyAsync", "launch"))}
+    last = max(k for k, r in enumerate(log) if r.startswith(("cudaMemcpyAsync", "launch",
+                                                             "cudaEventRecord")))
+    waited = {r.split()[1] for r in log[last:] if r.startswith("cudaStreamSynchronize")}
+    assert len(used) >= 2 and used <= waited
+    before = [o.copy() for o in out]
+    st, _ = host_fit(lib, ctx, data[:100], 100)
+    assert st == 0
+    for a, b in zip(before, out):
+        assert np.array_equal(a, b)
