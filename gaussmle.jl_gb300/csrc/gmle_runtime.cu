@@ -9,6 +9,7 @@
 // is copied out.  Device and pinned buffers grow on demand and are reused by
 // later calls; nothing the library allocates is handed to the caller.
 #include <cuda_runtime.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cmath>
@@ -288,13 +289,22 @@ gmle_status ensure_slot(gmle_ctx *ctx, Slot &s, int64_t rois, int64_t b2, bool n
     return GMLE_OK;
 }
 
-// Make the host own the pages of an output that the GPU will write: a page
-// of pageable memory first touched by the GPU could be placed in its memory.
-void touch_pages(void *p, size_t bytes)
+// Pageable memory that the copy engine is about to read or write itself: one access
+// per page by the host, which maps what is not resident yet (a file mapping, fresh
+// pages; a page first touched by the GPU would fault from there, one by one, and
+// could be placed in its memory).  The contents stay: an output's byte is written
+// back as it was, so that a call that fails later leaves its outputs alone.
+void map_input_pages(const void *p, size_t bytes, size_t page)
+{
+    const volatile char *c = static_cast<const volatile char *>(p);
+    for (size_t k = 0; k < bytes; k += page) (void)c[k];
+    if (bytes) (void)c[bytes - 1];
+}
+void map_output_pages(void *p, size_t bytes, size_t page)
 {
     volatile char *c = static_cast<volatile char *>(p);
-    for (size_t k = 0; k < bytes; k += 4096) c[k] = 0;
-    if (bytes) c[bytes - 1] = 0;
+    for (size_t k = 0; k < bytes; k += page) c[k] = c[k];
+    if (bytes) c[bytes - 1] = c[bytes - 1];
 }
 
 // Copy a finished slot's pinned outputs to the caller's pageable buffers.
@@ -494,16 +504,12 @@ gmle_status gmle_fit(gmle_ctx *ctx, const gmle_fit_desc *desc, const float *data
     // walks the host's page tables (GB300 beside its Grace CPU), any.  24 MB of
     // pageable pixels: 154 us copied directly; 1.4 ms by a host thread into the
     // pinned staging buffer and 0.13 ms from there.
-    const bool in_pinned = ctx->host_pages || is_pinned(data);
-    const bool out_pinned = ctx->host_pages || (is_pinned(params) && is_pinned(crlb) &&
-                                                is_pinned(llr) && (!flags || is_pinned(flags)));
+    const bool pinned_data = is_pinned(data), in_pinned = ctx->host_pages || pinned_data;
+    const bool pinned_out = is_pinned(params) && is_pinned(crlb) && is_pinned(llr) &&
+                            (!flags || is_pinned(flags));
+    const bool out_pinned = ctx->host_pages || pinned_out;
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
     const Tuning t = pick_tuning(ctx, desc, chunk);
-    if (ctx->host_pages) {
-        touch_pages(params, sizeof(float) * (size_t)n * P);
-        touch_pages(crlb, sizeof(float) * (size_t)n * P);
-        touch_pages(llr, sizeof(float) * (size_t)n);
-        if (flags) touch_pages(flags, (size_t)n);
-    }
 
     for (Slot &s : ctx->slots) {
         st = ensure_slot(ctx, s, chunk, b2, !(in_pinned && out_pinned));
@@ -523,6 +529,8 @@ gmle_status gmle_fit(gmle_ctx *ctx, const gmle_fit_desc *desc, const float *data
                 CK(cudaEventSynchronize(s.h2d_done), "cudaEventSynchronize");
                 std::memcpy(s.h_data, src, sizeof(float) * m * b2);
                 src = s.h_data;
+            } else if (!pinned_data) {
+                map_input_pages(src, sizeof(float) * m * b2, page);
             }
             CK(cudaMemcpyAsync(s.data, src, sizeof(float) * m * b2, cudaMemcpyHostToDevice, ctx->s_h2d),
                "H2D data");
@@ -539,6 +547,12 @@ gmle_status gmle_fit(gmle_ctx *ctx, const gmle_fit_desc *desc, const float *data
             CK(launch(ctx, desc, a, t.rois_per_block, ctx->s_fit), "fit kernel launch");
             CK(cudaEventRecord(s.fit_done, ctx->s_fit), "cudaEventRecord");
             CK(cudaStreamWaitEvent(ctx->s_d2h, s.fit_done, 0), "cudaStreamWaitEvent");
+            if (out_pinned && !pinned_out) {  // (while the chunk is copied in and fitted)
+                map_output_pages(params + off * P, sizeof(float) * m * P, page);
+                map_output_pages(crlb + off * P, sizeof(float) * m * P, page);
+                map_output_pages(llr + off, sizeof(float) * m, page);
+                if (flags) map_output_pages(flags + off, m, page);
+            }
             float *op = out_pinned ? params + off * P : s.h_params;
             float *oc = out_pinned ? crlb + off * P : s.h_crlb;
             float *ol = out_pinned ? llr + off : s.h_llr;

@@ -94,3 +94,32 @@ def test_a_failed_fit_leaves_nothing_behind(lib, ctx, host_pages, name, nth):
     assert st == 0
     for a, b in zip(before, out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("name", ["cudaMalloc", "cudaEventCreateWithFlags", "cudaMemcpyAsync"])
+def test_a_fit_that_fails_before_its_results_leaves_the_outputs_alone(lib, ctx, name):
+    """Where the GPU takes pageable memory as it is, its pages are mapped by the host
+    first: without a change to the outputs, which hold the caller's values until results
+    come."""
+    lib.gmle_destroy(ctx)
+    lib.fake_host_pages(1)
+    assert lib.gmle_create(C.byref(ctx), 0) == 0
+    data = np.zeros((40_000, BOX * BOX), np.float32)
+    lib.fake_fail(name.encode(), 1)
+    st, out = host_fit(lib, ctx, data, len(data))
+    assert st != 0
+    for o in out:
+        assert (o == 7).all()
+    st, out = host_fit(lib, ctx, data, len(data))
+    assert st == 0 and (out[0] == 0).all()  # (the fake's results: zeros)
+
+
+def test_inputs_that_are_not_resident(lib, ctx, tmp_path):
+    """A read-only file mapping as input, as raw movies often are."""
+    lib.gmle_destroy(ctx)
+    lib.fake_host_pages(1)
+    assert lib.gmle_create(C.byref(ctx), 0) == 0
+    np.zeros((3000, BOX * BOX), np.float32).tofile(tmp_path / "rois.bin")
+    m = np.memmap(tmp_path / "rois.bin", np.float32, "r", shape=(3000, BOX * BOX))
+    st, out = host_fit(lib, ctx, m, len(m))
+    assert st == 0 and (out[0] == 0).all()
