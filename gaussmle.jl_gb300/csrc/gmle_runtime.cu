@@ -973,21 +973,13 @@ gmle_status enqueue_table_launch(gmle_ctx *ctx, MixedSet &m, const TableLaunch &
     return GMLE_OK;
 }
 
-int plan_stream(int index, bool holds_tmem, int nf)
-{
-    // Persistent launches whose kernel holds tensor memory run in sequence on
-    // fork 0: a persistent CTA keeps its columns until its launch runs out of
-    // tiles, so a concurrent one's CTAs would wait in tcgen05.alloc on the
-    // same SMs.  The others spread over the remaining forks.
-    if (nf <= 1 || holds_tmem) return 0;
-    return 1 + index % (nf - 1);
-}
-
 gmle_status enqueue_plan(gmle_ctx *ctx, MixedSet &m, const MixedPlan &plan, cudaStream_t s)
 {
     // The launches of a plan (plain launches of large groups, table launches
-    // of the rest) run concurrently on the fork streams, joined back into s,
-    // so that each launch's last, partly filled wave overlaps the others.
+    // of the rest with one block per tile) run concurrently on the fork streams,
+    // joined back into s, so that each launch's last, partly filled wave overlaps
+    // the others.  None is persistent: a CTA frees its tensor memory after its
+    // tile, so they overlap freely.
     const int np = (int)plan.plain.size(), nl = (int)plan.launches.size();
     const int units = np + nl;
     const bool fork = units > 1;
@@ -1002,16 +994,13 @@ gmle_status enqueue_plan(gmle_ctx *ctx, MixedSet &m, const MixedPlan &plan, cuda
         const Tuning t = pick_tuning(ctx, &G.desc, G.n);
         KernelArgs a = make_args(ctx, &G.desc, G.data, G.x_corners, G.y_corners, G.n, G.params,
                                  G.crlb, G.llr, G.flags, t.tpr);
-        // plain launches are not persistent (a CTA frees its tensor memory
-        // after one tile), so they overlap freely
         CK(launch(ctx, &G.desc, a, t.rois_per_block, fork ? m.fork[u % nf] : s),
            "fit kernel launch");
     }
     for (int l = 0; l < nl; l++) {
         const TableLaunch &L = plan.launches[l];
-        const bool tm = L.persistent && holds_tmem(L.scmos, L.shape.tpr);
-        const gmle_status st = enqueue_table_launch(
-            ctx, m, L, fork ? m.fork[plan_stream(np + l, tm, nf)] : s);
+        const gmle_status st =
+            enqueue_table_launch(ctx, m, L, fork ? m.fork[(np + l) % nf] : s);
         if (st != GMLE_OK) return st;
     }
     for (int f = 0; f < nf; f++) {

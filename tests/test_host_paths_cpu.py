@@ -9,10 +9,11 @@ import numpy as np
 import pytest
 
 from conftest import ROOT
-from gaussmle_gb300 import build
+from gaussmle_gb300 import _lib, build, serve
 from gaussmle_gb300.constraints import default_constraints
 from gaussmle_gb300.fitter import make_desc
-from gaussmle_gb300.models import GaussianXYNB
+from gaussmle_gb300.models import (AstigmaticXYZNB, GaussianXYNB, GaussianXYNBS,
+                                   GaussianXYNBSXSY)
 
 SMS = 152
 
@@ -123,3 +124,32 @@ def test_inputs_that_are_not_resident(lib, ctx, tmp_path):
     m = np.memmap(tmp_path / "rois.bin", np.float32, "r", shape=(3000, BOX * BOX))
     st, out = host_fit(lib, ctx, m, len(m))
     assert st == 0 and (out[0] == 0).all()
+
+
+PSF = {0: GaussianXYNB(1.3), 1: GaussianXYNBS(), 2: GaussianXYNBSXSY(),
+       3: AstigmaticXYZNB(1.3, 1.3, 0.05, 0.05, 0.3, 0.3, 50.0, 100.0)}
+
+
+def groups(kinds):
+    """gmle_group array of (model, box, n); the fake's kernels read and write nothing."""
+    some = np.zeros(1, np.float32)
+    gs = []
+    for model, box, n in kinds:
+        g = serve.make_group(PSF[model], box, 0, default_constraints(PSF[model], box), some, some,
+                             some, np.empty((n, 6), np.float32), some, some)
+        gs.append(g)
+    return (_lib.Group * len(gs))(*gs)
+
+
+@pytest.mark.parametrize("kinds", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("large", [0, 1])
+def test_the_launches_of_a_submission_take_every_stream(lib, ctx, kinds, large):
+    """One launch per kind (a group of 65536 ROIs or more: its own), each on a stream of
+    its own up to four; a single launch on the caller's."""
+    gs = groups([(k % 4, 7 + k, 70_000 if k < large else 500) for k in range(kinds)])
+    lib.fake_clear()
+    assert lib.gmle_fit_mixed_device(ctx, gs, len(gs), C.c_void_p(999)) == 0
+    streams = [c[0] for c in calls(lib, "launch")]
+    assert len(streams) == kinds
+    assert len(set(streams)) == min(kinds, 4)
+    assert (streams == [999]) if kinds == 1 else (999 not in streams)
