@@ -213,19 +213,23 @@ extern "C" gmle_status gmle_fit_mixed_device_noalloc(const gmle_group *groups, i
     KernelArgs *h_args = reinterpret_cast<KernelArgs *>(g_stage + kArgsOff);
     unsigned long long *d_counters = reinterpret_cast<unsigned long long *>(S.scratch + kCountersOff);
     int used = 0;
-    int64_t together = 0;
-    for (int k = 0; k < ngroups; k++) together += std::max<int64_t>(groups[k].n, 0);
     int first[kKinds] = {};
     gmle::LaunchShape shape[kKinds] = {};
     for (int kind = 0; kind < kKinds; kind++) {
         int cnt = 0;
+        int64_t rois = 0;
         for (int k = 0; k < ngroups; k++)
-            if (groups[k].n > 0 && gmle_rt::kind_of(groups[k].desc) == kind) g_order[cnt++] = k;
+            if (groups[k].n > 0 && gmle_rt::kind_of(groups[k].desc) == kind) {
+                g_order[cnt++] = k;
+                rois += groups[k].n;
+            }
         first[kind] = used;
         if (cnt == 0) continue;
         const gmle_fit_desc &d0 = groups[g_order[0]].desc;
         const bool scmos = d0.camera != GMLE_CAMERA_POISSON;
-        const gmle_rt::Tuning t = gmle_rt::default_tuning(S.num_sms, d0.model, d0.box, scmos, together, together);
+        // The kinds' launches follow one another on the caller's stream, each with the
+        // GPU to itself: a shape by the kind's own ROIs.
+        const gmle_rt::Tuning t = gmle_rt::default_tuning(S.num_sms, d0.model, d0.box, scmos, rois);
         int64_t tiles = 0;
         for (int q = 0; q < cnt; q++) {
             const gmle_group &G = groups[g_order[q]];

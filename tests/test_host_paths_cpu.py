@@ -153,3 +153,24 @@ def test_the_launches_of_a_submission_take_every_stream(lib, ctx, kinds, large):
     assert len(streams) == kinds
     assert len(set(streams)) == min(kinds, 4)
     assert (streams == [999]) if kinds == 1 else (999 not in streams)
+
+
+@pytest.mark.parametrize("n,threads,grid", [
+    (300, 32, 300),          # a warp per ROI, a ROI per block
+    (5_000, 128, 157),       # four lanes, 32 ROIs per block
+    (100_000, 64, 4 * SMS),  # one thread, as many blocks as are resident (the fake's four per SM)
+])
+def test_the_launches_without_allocation_go_by_their_own_kinds_rois(lib, n, threads, grid):
+    """gmle_fit_mixed_device_noalloc's launches run one after another, so that a kind's
+    shape does not depend on what else the call holds."""
+    err = C.create_string_buffer(256)
+    shapes = []
+    for others in ([], [(1, 9, 200_000)], [(1, 9, 40)]):
+        gs = groups([(0, 11, n)] + others)
+        lib.fake_clear()
+        assert lib.gmle_fit_mixed_device_noalloc(gs, len(gs), None, None, None, 0, 0,
+                                                 C.c_void_p(999), err, 256) == 0, err.value
+        fits = [c for c in calls(lib, "launch") if c[1:3] != (1, 256)]  # (without the table writes)
+        assert len(fits) == len(gs) and all(c[0] == 999 for c in fits)
+        shapes.append(fits[0][1:3])
+    assert shapes == [(grid, threads)] * 3
