@@ -36,8 +36,7 @@ inline bool box_supported(int box) { return box_index(box) >= 0; }
 // The part of the odd boxes 5..15 (the most used sizes, with 8-lane kernels).
 __host__ __device__ constexpr bool main_box(int box) { return box >= 5 && box <= 15 && (box & 1); }
 
-// Largest block of the one-thread-per-ROI kernel that can be asked for (the
-// default for large sCMOS batches may be r1_scmos_threads).
+// Largest block of the one-thread-per-ROI kernel (16x16 sCMOS: r1_scmos_threads).
 constexpr int kMaxThreadsR1 = 128;
 
 // One launch of a model's kernel.  Plain (t.header == nullptr): ceil(a.n / rpb)

@@ -307,6 +307,12 @@ void map_output_pages(void *p, size_t bytes, size_t page)
     if (bytes) c[bytes - 1] = c[bytes - 1];
 }
 
+// Largest block of the one-thread-per-ROI kernel.
+int max_threads_r1(int box, bool scmos)
+{
+    return scmos ? std::max(gmle::kMaxThreadsR1, gmle::r1_scmos_threads(box)) : gmle::kMaxThreadsR1;
+}
+
 // Copy a finished slot's pinned outputs to the caller's pageable buffers.
 gmle_status flush_slot(gmle_ctx *ctx, Slot &s)
 {
@@ -595,9 +601,12 @@ gmle_status gmle_get_tuning(gmle_ctx *ctx, int32_t model, int32_t box, int32_t c
     if (!ctx || !threads_per_roi || !rois_per_block) return GMLE_INVALID_ARG;
     std::lock_guard<std::mutex> lk(ctx->mu);
     const bool scmos = camera != GMLE_CAMERA_POISSON;
+    const int64_t many = 1ll << 40;
     auto it = ctx->tuning.find({model, box, (int)scmos});
     Tuning t = it != ctx->tuning.end() ? it->second
-                                       : default_tuning(ctx->num_sms, model, box, scmos, 1ll << 40);
+               : gmle::large_box(box)
+                   ? Tuning{32, gmle::warp_rois_per_block(ctx->num_sms, box, scmos, many)}
+                   : default_tuning(ctx->num_sms, model, box, scmos, many);
     *threads_per_roi = t.tpr;
     *rois_per_block = t.rois_per_block;
     return GMLE_OK;
@@ -621,10 +630,10 @@ gmle_status gmle_set_tuning(gmle_ctx *ctx, int32_t model, int32_t box, int32_t c
                     "threads_per_roi must be 1, 2, 4, or 8 (2 and 8: odd boxes 5..15 only)");
     const bool scmos = camera != GMLE_CAMERA_POISSON;
     const int threads = tpr * rois_per_block;
-    if (rois_per_block < 1 || threads > (tpr == 1 ? gmle::kMaxThreadsR1 : 256) || threads % 32)
+    const int most = tpr > 1 ? 256 : max_threads_r1(box, scmos);
+    if (rois_per_block < 1 || threads > most || threads % 32)
         return fail(ctx, GMLE_INVALID_ARG,
-                    "threads_per_roi * rois_per_block must be a multiple of 32, at most 256 "
-                    "(64 with one thread per ROI)");
+                    "threads_per_roi * rois_per_block must be a multiple of 32, at most %d", most);
     if (gmle::smem_bytes(model, box, scmos, tpr, rois_per_block) > 227 * 1024)
         return fail(ctx, GMLE_INVALID_ARG, "launch shape needs more than 227 KiB shared memory");
     ctx->tuning[{model, box, (int)scmos}] = {tpr, rois_per_block};

@@ -169,8 +169,11 @@ gmle_status gmle_fit_device_errors(gmle_ctx *ctx, int64_t *count);
  * ROIs per block, as picked by the autotuner (or set by gmle_set_tuning;
  * setting (0, 0) forgets the entry and restores the size-based default).
  * Threads per ROI: 1, 2, 4, or 8 (2 and 8 for odd boxes 5..15 only); one thread per
- * ROI allows at most 128 ROIs per block, several lanes 256 threads per block.
- * Boxes 3..16; larger boxes run in one fixed shape.
+ * ROI allows at most 128 ROIs per block (224 for 16x16 sCMOS), several lanes 256
+ * threads per block.  Boxes 3..16; larger boxes run in one fixed shape, a warp (32
+ * threads) per ROI.  Without an entry gmle_get_tuning answers the default of large
+ * batches; the default itself follows the batch's size (a warp per ROI for the
+ * smallest, then four lanes, then one thread).
  */
 gmle_status gmle_get_tuning(gmle_ctx *ctx, int32_t model, int32_t box, int32_t camera,
                             int32_t *threads_per_roi, int32_t *rois_per_block);

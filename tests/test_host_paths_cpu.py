@@ -174,3 +174,41 @@ def test_the_launches_without_allocation_go_by_their_own_kinds_rois(lib, n, thre
         assert len(fits) == len(gs) and all(c[0] == 999 for c in fits)
         shapes.append(fits[0][1:3])
     assert shapes == [(grid, threads)] * 3
+
+
+def get_tuning(lib, ctx, model, box, camera):
+    t, r = C.c_int32(), C.c_int32()
+    assert lib.gmle_get_tuning(ctx, model, box, camera, C.byref(t), C.byref(r)) == 0
+    return t.value, r.value
+
+
+def test_every_launch_shape_that_is_answered_can_be_set(lib, ctx):
+    """A program that saves the shapes and sets them again: for every specialised box,
+    and back to the default."""
+    for model in range(4):
+        for camera in range(3):
+            for box in range(3, 17):
+                shape = get_tuning(lib, ctx, model, box, camera)
+                assert lib.gmle_set_tuning(ctx, model, box, camera, *shape) == 0, (
+                    model, box, camera, shape, lib.gmle_last_error(ctx))
+                assert get_tuning(lib, ctx, model, box, camera) == shape
+                assert lib.gmle_set_tuning(ctx, model, box, camera, 0, 0) == 0
+
+
+@pytest.mark.parametrize("box,camera,most", [(16, 1, 224), (16, 2, 224), (16, 0, 128), (15, 1, 128),
+                                             (11, 2, 128)])
+def test_one_thread_blocks_end_where_the_kernel_does(lib, ctx, box, camera, most):
+    assert lib.gmle_set_tuning(ctx, 0, box, camera, 1, most) == 0
+    assert lib.gmle_set_tuning(ctx, 0, box, camera, 1, most + 32) == 1
+    assert str(most).encode() in lib.gmle_last_error(ctx)
+
+
+@pytest.mark.parametrize("box", [17, 21, 33, 64])
+def test_large_boxes_answer_the_shape_they_run_in(lib, ctx, box):
+    n, some = 3000, np.zeros(1, np.float32)
+    lib.fake_clear()
+    assert lib.gmle_fit_device(ctx, C.byref(desc(box)), p(some), None, None, C.c_int64(n), p(some),
+                               p(some), p(some), None, C.c_void_p(7)) == 0
+    _, grid, threads, _ = calls(lib, "launch")[0]
+    tpr, rpb = get_tuning(lib, ctx, 0, box, 0)
+    assert tpr == 32 and threads == 32 * rpb and grid == -(-n // rpb)
