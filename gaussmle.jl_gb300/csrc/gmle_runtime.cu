@@ -687,51 +687,63 @@ gmle_status gmle_autotune(gmle_ctx *ctx, const gmle_fit_desc *desc, const float 
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0), "cudaEventCreate");
     CK(cudaEventCreate(&e1), "cudaEventCreate");
-    Tuning best{0, 0};
-    float best_ms = 1e30f;
-    // threads per block: powers of two, and for one thread per ROI also 96
-    // (three warps: two such blocks of large sCMOS ROIs fit where one of four
-    // warps does)
-    static const int kThreads[] = {32, 64, 96, 128, 256};
+    // Threads per block: powers of two, and for one thread per ROI also 96 (three
+    // warps: two such blocks of large sCMOS ROIs fit where one of four warps does) and
+    // the 224 of 16x16 sCMOS.
+    std::vector<Tuning> shapes;
     for (int tpr : {1, 2, 4, 8}) {
         if (!gmle::tpr_supported(tpr, desc->box)) continue;
-        for (int threads : kThreads) {
-            if (threads > (tpr == 1 ? gmle::kMaxThreadsR1 : 256)) continue;
-            if (tpr > 1 && threads == 96) continue;
+        for (int threads : {32, 64, 96, 128, 224, 256}) {
+            if (threads > (tpr == 1 ? max_threads_r1(desc->box, scmos) : 256)) continue;
+            if (threads % 64 == 32 && threads > 32 && tpr > 1) continue;
             const int rpb = threads / tpr;
             if (rpb < 1 || gmle::smem_bytes(desc->model, desc->box, scmos, tpr, rpb) > 227 * 1024)
                 continue;
-            KernelArgs a = make_args(ctx, desc, d_data, d_x_corners, d_y_corners, n, d_params,
-                                     d_crlb, d_llr, d_flags, tpr);
-            // two warm-up launches, then the fastest of four timed one by one:
-            // a single average was swayed by clock ramps and by other work on
-            // the GPU, and picked slower shapes
-            cudaError_t e = launch(ctx, desc, a, rpb, ctx->s_fit);
-            if (e == cudaSuccess) e = launch(ctx, desc, a, rpb, ctx->s_fit);
-            float ms = 1e30f;
-            for (int rep = 0; rep < 4 && e == cudaSuccess; rep++) {
-                e = cudaEventRecord(e0, ctx->s_fit);
-                if (e == cudaSuccess) e = launch(ctx, desc, a, rpb, ctx->s_fit);
-                if (e == cudaSuccess) e = cudaEventRecord(e1, ctx->s_fit);
-                if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-                float t = 0.f;
-                if (e == cudaSuccess) e = cudaEventElapsedTime(&t, e0, e1);
-                if (e == cudaSuccess) ms = std::min(ms, t);
-            }
-            if (e != cudaSuccess) {
-                cudaEventDestroy(e0);
-                cudaEventDestroy(e1);
-                return cuda_fail(ctx, e, "autotune launch");
-            }
-            if (ms < best_ms) {
-                best_ms = ms;
-                best = {tpr, rpb};
-            }
+            shapes.push_back({tpr, rpb});
+        }
+    }
+    // A warp per ROI is the default of the smallest batches only: it is timed where it
+    // is this one's, and nothing is kept where it wins (larger batches of the kind would
+    // take several times as long; XYNB 11x11, 200 ROIs: 21 us, 37 in the fastest of the
+    // other shapes).
+    const Tuning usual = default_tuning(ctx->num_sms, desc->model, desc->box, scmos, n);
+    if (usual.tpr == 32) shapes.push_back(usual);
+    Tuning best{0, 0};
+    float best_ms = 1e30f;
+    for (const Tuning &shape : shapes) {
+        KernelArgs a = make_args(ctx, desc, d_data, d_x_corners, d_y_corners, n, d_params,
+                                 d_crlb, d_llr, d_flags, shape.tpr);
+        // two warm-up launches, then the fastest of four timed one by one:
+        // a single average was swayed by clock ramps and by other work on
+        // the GPU, and picked slower shapes
+        cudaError_t e = launch(ctx, desc, a, shape.rois_per_block, ctx->s_fit);
+        if (e == cudaSuccess) e = launch(ctx, desc, a, shape.rois_per_block, ctx->s_fit);
+        float ms = 1e30f;
+        for (int rep = 0; rep < 4 && e == cudaSuccess; rep++) {
+            e = cudaEventRecord(e0, ctx->s_fit);
+            if (e == cudaSuccess) e = launch(ctx, desc, a, shape.rois_per_block, ctx->s_fit);
+            if (e == cudaSuccess) e = cudaEventRecord(e1, ctx->s_fit);
+            if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+            float t = 0.f;
+            if (e == cudaSuccess) e = cudaEventElapsedTime(&t, e0, e1);
+            if (e == cudaSuccess) ms = std::min(ms, t);
+        }
+        if (e != cudaSuccess) {
+            cudaEventDestroy(e0);
+            cudaEventDestroy(e1);
+            return cuda_fail(ctx, e, "autotune launch");
+        }
+        if (ms < best_ms) {
+            best_ms = ms;
+            best = shape;
         }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    ctx->tuning[{desc->model, desc->box, (int)scmos}] = best;
+    if (best.tpr == 32)
+        ctx->tuning.erase({desc->model, desc->box, (int)scmos});
+    else
+        ctx->tuning[{desc->model, desc->box, (int)scmos}] = best;
     if (threads_per_roi) *threads_per_roi = best.tpr;
     if (rois_per_block) *rois_per_block = best.rois_per_block;
     if (ms_per_fit) *ms_per_fit = best_ms;

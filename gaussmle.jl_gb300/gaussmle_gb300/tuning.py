@@ -51,7 +51,8 @@ def load_cache(ctx: _lib.Context) -> int:
 
 def autotune(ctx: _lib.Context, desc: _lib.FitDesc, data, xc, yc, params, crlb, llr,
              flags=None, save: bool = True) -> tuple[int, int, float]:
-    """Time all launch shapes on the given CUDA tensors; keep and cache the best."""
+    """Time all launch shapes on the given CUDA tensors; keep and cache the best
+    (a warp per ROI, 32 threads, is a default of the smallest batches and is not kept)."""
     t, r, ms = C.c_int32(), C.c_int32(), C.c_float()
     p = lambda x: C.c_void_p(x.data_ptr()) if x is not None else None
     ctx.check(ctx.lib.gmle_autotune(ctx.handle, C.byref(desc), p(data), p(xc), p(yc),
@@ -61,8 +62,12 @@ def autotune(ctx: _lib.Context, desc: _lib.FitDesc, data, xc, yc, params, crlb, 
         try:
             CACHE.parent.mkdir(parents=True, exist_ok=True)
             allt = json.loads(CACHE.read_text()) if CACHE.exists() else {}
-            allt.setdefault(_gpu_name(ctx.device), {})[
-                _key(desc.model, desc.box, desc.camera)] = [t.value, r.value]
+            table = allt.setdefault(_gpu_name(ctx.device), {})
+            key = _key(desc.model, desc.box, desc.camera)
+            if t.value == 32:
+                table.pop(key, None)
+            else:
+                table[key] = [t.value, r.value]
             CACHE.write_text(json.dumps(allt, indent=1))
         except OSError:
             pass

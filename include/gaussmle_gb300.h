@@ -182,10 +182,13 @@ gmle_status gmle_set_tuning(gmle_ctx *ctx, int32_t model, int32_t box, int32_t c
 
 /*
  * Autotuner: times every candidate launch shape (threads per ROI 1, 2, 4, 8;
- * 32..256 threads per block, within 227 KiB of shared memory) of the fit
+ * 32..256 threads per block, within 227 KiB of shared memory; a warp per ROI where
+ * that is the default of such a batch) of the fit
  * kernel for `desc` on a device-resident batch, keeps the fastest for
  * (model, box, camera family) in the context and returns it with its time
- * per launch.  The output buffers are overwritten.  No reference counterpart:
+ * per launch.  Where a warp per ROI is the fastest it is returned (32 threads), but
+ * no shape is kept: the kind goes by its default, which for such batches is that one.
+ * Boxes above 16 have one shape, a warp per ROI.  The output buffers are overwritten.  No reference counterpart:
  * KernelAbstractions picks the reference's workgroup size.
  */
 gmle_status gmle_autotune(gmle_ctx *ctx, const gmle_fit_desc *desc, const float *d_data,

@@ -5,6 +5,7 @@
 // (tests/test_host_paths_cpu.py).
 #include <cuda_runtime_api.h>
 
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <map>
@@ -14,6 +15,7 @@ namespace {
 
 std::string g_log, g_fail_name;
 int g_fail_in = 0, g_host_pages = 0, g_next = 0;
+float g_fast_grid = 0, g_fast_block = 0;
 std::map<const void *, size_t> g_pinned;
 cudaError_t g_last = cudaSuccess;  // a launch's error, read by cudaGetLastError
 struct Config { dim3 grid, block; size_t smem; cudaStream_t stream; } g_config;
@@ -49,6 +51,7 @@ FAKE void fake_pin(const void *p, size_t bytes, int on)
     if (on) g_pinned[p] = bytes;
     else g_pinned.erase(p);
 }
+FAKE void fake_fastest(int grid, int block) { g_fast_grid = (float)grid; g_fast_block = (float)block; }
 // The calls since the last fake_clear, one per line: name, stream, and for a launch its
 // grid, block and dynamic shared memory.
 FAKE const char *fake_log() { return g_log.c_str(); }
@@ -159,10 +162,11 @@ FAKE cudaError_t cudaEventDestroy(cudaEvent_t) { return called("cudaEventDestroy
 FAKE cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t s) { return called("cudaEventRecord", s); }
 FAKE cudaError_t cudaEventSynchronize(cudaEvent_t) { return called("cudaEventSynchronize"); }
 FAKE cudaError_t cudaEventQuery(cudaEvent_t) { return cudaSuccess; }
-// A launch takes a millisecond for each of its blocks' threads (threads 32: 32 ms).
+// A launch takes as many ms as its grid and block differ from fake_fastest's.
 FAKE cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t)
 {
-    *ms = (float)g_config.block.x;
+    *ms = 1.0f + std::abs((float)g_config.block.x - g_fast_block) +
+          std::abs((float)g_config.grid.x - g_fast_grid);
     return called("cudaEventElapsedTime");
 }
 FAKE cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaErrorUnknown; }

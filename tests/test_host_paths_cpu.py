@@ -212,3 +212,68 @@ def test_large_boxes_answer_the_shape_they_run_in(lib, ctx, box):
     _, grid, threads, _ = calls(lib, "launch")[0]
     tpr, rpb = get_tuning(lib, ctx, 0, box, 0)
     assert tpr == 32 and threads == 32 * rpb and grid == -(-n // rpb)
+
+
+def autotune(lib, ctx, box, camera, n, grid, threads):
+    """Autotune where the launch of that grid and block is the fastest; (shape, kept)."""
+    some, d = np.ones(4, np.float32), desc(box)
+    d.camera = camera
+    lib.fake_fastest(grid, threads)
+    t, r, ms = C.c_int32(), C.c_int32(), C.c_float()
+    if camera:
+        assert lib.gmle_set_calibration(ctx, p(np.ones((64, 64), np.float32)), None, None, 64, 64) == 0
+    st = lib.gmle_autotune(ctx, C.byref(d), p(some), p(some), p(some), C.c_int64(n), p(some), p(some),
+                           p(some), None, C.byref(t), C.byref(r), C.byref(ms))
+    assert st == 0, lib.gmle_last_error(ctx)
+    lib.fake_clear()
+    assert lib.gmle_fit_device(ctx, C.byref(d), p(some), p(some), p(some), C.c_int64(n), p(some),
+                               p(some), p(some), None, C.c_void_p(7)) == 0
+    _, g, b, _ = calls(lib, "launch")[0]
+    return (t.value, r.value, ms.value), (g, b)
+
+
+@pytest.mark.parametrize("box,camera,n,grid,threads,tpr", [
+    (11, 0, 200, 200, 32, 32),        # a warp per ROI, the default of 200 ROIs
+    (11, 0, 200, 25, 32, 4),          # another shape, where it is faster
+    (16, 1, 100_000, 447, 224, 1),    # the blocks of large 16x16 sCMOS batches
+    (16, 1, 100_000, 1042, 96, 1),
+    (16, 0, 100_000, 1563, 64, 1)])
+def test_autotune_times_the_default_shape_too(lib, ctx, box, camera, n, grid, threads, tpr):
+    """The shape that a batch runs in afterwards is the fastest, also where that is the
+    shape it would have had anyway."""
+    (t, r, ms), ran = autotune(lib, ctx, box, camera, n, grid, threads)
+    assert (t, t * r, ms) == (tpr, threads, 1.0) and ran == (grid, threads)
+    if t == 32:  # not kept for the larger batches of the kind
+        assert get_tuning(lib, ctx, 0, box, camera)[0] == 1
+    else:
+        assert get_tuning(lib, ctx, 0, box, camera) == (t, r)
+
+
+def test_autotune_saves_no_shape_of_the_smallest_batches(tmp_path, monkeypatch):
+    import json
+    from gaussmle_gb300 import tuning
+    monkeypatch.setattr(tuning, "CACHE", tmp_path / "tuning.json")
+    monkeypatch.setattr(tuning, "_gpu_name", lambda device: "GB300")
+
+    class Tensor:
+        shape = (200, 4)
+
+        def data_ptr(self):
+            return 0
+
+    class Ctx:
+        handle, device, lib, shape = None, 0, None, None
+
+        def gmle_autotune(self, *a):
+            for q, v in zip(a[-3:], self.shape + (0.1,)):
+                q._obj.value = v
+            return 0
+
+        def check(self, st):
+            assert st == 0
+
+    ctx, x = Ctx(), Tensor()
+    ctx.lib = ctx
+    for ctx.shape, want in [((1, 64), {"0/11/0": [1, 64]}), ((32, 1), {}), ((32, 4), {})]:
+        assert tuning.autotune(ctx, desc(11), x, None, None, x, x, x)[:2] == ctx.shape
+        assert json.loads(tuning.CACHE.read_text())["GB300"] == want
