@@ -150,10 +150,9 @@ int nparams(int model);
 
 gmle_status init_mixed_set(gmle_ctx *ctx, MixedSet &m);
 void free_mixed_set(MixedSet &m);
-// ROIs per SM up to which a warp fits a ROI (alone, and of a submission whose
-// launches share the GPU), and from which one thread does in such a submission
-// (default_tuning).
-constexpr int kWarpLine = 20, kWarpTogether = 20, kSubmissionLine = 200;
+// ROIs per SM below which a warp fits a ROI, and from which one thread does in a
+// submission whose launches share the GPU (default_tuning).
+constexpr int kWarpLine = 20, kSubmissionLine = 200;
 // How a table launch picks its shape: from the context's tuning for the kind,
 // else the size-based default for a submission of `shape_rois` ROIs (0: this
 // one's); with request_rois > 0 by each group's own size instead, so that

@@ -213,6 +213,8 @@ extern "C" gmle_status gmle_fit_mixed_device_noalloc(const gmle_group *groups, i
     KernelArgs *h_args = reinterpret_cast<KernelArgs *>(g_stage + kArgsOff);
     unsigned long long *d_counters = reinterpret_cast<unsigned long long *>(S.scratch + kCountersOff);
     int used = 0;
+    int64_t together = 0;
+    for (int k = 0; k < ngroups; k++) together += std::max<int64_t>(groups[k].n, 0);
     int first[kKinds] = {};
     gmle::LaunchShape shape[kKinds] = {};
     for (int kind = 0; kind < kKinds; kind++) {
@@ -228,8 +230,13 @@ extern "C" gmle_status gmle_fit_mixed_device_noalloc(const gmle_group *groups, i
         const gmle_fit_desc &d0 = groups[g_order[0]].desc;
         const bool scmos = d0.camera != GMLE_CAMERA_POISSON;
         // The kinds' launches follow one another on the caller's stream, each with the
-        // GPU to itself: a shape by the kind's own ROIs.
-        const gmle_rt::Tuning t = gmle_rt::default_tuning(S.num_sms, d0.model, d0.box, scmos, rois);
+        // GPU to itself: a shape by the kind's own ROIs.  But a warp per ROI only where
+        // gmle_fit_mixed_device would take it, for a call that is small as a whole: the
+        // small kinds of a larger call then have its four lanes, and the same bits, up to
+        // 200 ROIs per SM in all (an ill-posed astigmatic fit can end elsewhere by an ulp).
+        const int64_t line = (int64_t)gmle_rt::kWarpLine * S.num_sms;
+        const gmle_rt::Tuning t = gmle_rt::default_tuning(
+            S.num_sms, d0.model, d0.box, scmos, together < line ? rois : std::max(rois, line));
         int64_t tiles = 0;
         for (int q = 0; q < cnt; q++) {
             const gmle_group &G = groups[g_order[q]];

@@ -91,11 +91,13 @@ namespace gmle_rt {
 // lanes at 32 / 64 / 96 ROIs per SM, one thread up to 128): XYNB 11x11 37 / 45 / 53,
 // 60; 11x11 sCMOS 42 / 49 / 60, 64; XYNBS 9x9 41 / 49 / 60, 54; XYNBS 13x13 sCMOS
 // 56 / 70 / 88, 86; astigmatic 15x15 66 / 83 / 108, 105.  So the line is two warps per
-// scheduler; three where they still win, which takes a model with few sums (XYNB from
-// 8 pixels on; 9x9, split 5 + 4, does not: 48 and 46) or XYNBS 11x11 (64 and 70) and
-// 12x12 (74 and 87 with sCMOS; a few other boxes would gain up to 10 %); one for 3x3 and 5x5, which the lanes split most
-// unevenly (XYNBS 5x5 39 at 64, 35).  Of 16x16 sCMOS a third block does not fit the SM
-// (171 and 125), nor of the astigmatic 13x13 (134 and 92).
+// scheduler, but for what was measured otherwise, box by box: three where they win by
+// more than the runs differ, i.e. XYNB from 8 pixels on (few sums per pixel; 9x9, split
+// 5 + 4, does not: 48 and 46) and XYNBS 11x11 (64 and 70) and 12x12 (74 and 87 with
+// sCMOS) - a few other boxes would gain up to 10 % and keep two; one for 3x3 and 5x5, which
+// the lanes split most unevenly (XYNBS 5x5 39 at 64, 35).  Of 16x16 sCMOS a third
+// block does not fit the SM (171 and 125), nor of the astigmatic 13x13 (134 and 92).
+// A box's line can only be found by measuring it: no formula in box and model gives these.
 static int plain_line(int model, int box, bool scmos)
 {
     if (box == 3 || box == 5) return 32;
@@ -136,7 +138,7 @@ static int plain_line(int model, int box, bool scmos)
 Tuning default_tuning(int num_sms, int model, int box, bool scmos, int64_t n, int64_t together)
 {
     const int64_t all = together > 0 ? together : n;
-    if (all < (int64_t)(together > 0 ? kWarpTogether : kWarpLine) * num_sms)
+    if (all < (int64_t)kWarpLine * num_sms)
         return {32, gmle::warp_rois_per_block(num_sms, box, scmos, all)};
     if (together > 0 ? all < (int64_t)kSubmissionLine * num_sms
                      : n <= (int64_t)plain_line(model, box, scmos) * num_sms)
@@ -752,7 +754,7 @@ gmle_status gmle_autotune(gmle_ctx *ctx, const gmle_fit_desc *desc, const float 
 
 }  // extern "C"
 
-// ---- mixed batches: one persistent table launch per (family, model, box) ----------
+// ---- mixed batches: one table launch per (family, model, box) ---------------------
 
 namespace gmle_rt {
 
@@ -889,7 +891,7 @@ gmle_status plan_mixed(gmle_ctx *ctx, const gmle_group *groups, int32_t ngroups,
         L.scmos = d0.camera != GMLE_CAMERA_POISSON;
         const int64_t all =
             opt.request_rois > 0
-                ? (int64_t)(table >= kKinds ? kSubmissionLine : kWarpTogether) * ctx->num_sms
+                ? (int64_t)(table >= kKinds ? kSubmissionLine : kWarpLine) * ctx->num_sms
             : opt.shape_rois > 0 ? opt.shape_rois : together;
         const Tuning t = pick_tuning(ctx, &d0, all, all);
         const int rpb = t.rois_per_block;

@@ -156,24 +156,43 @@ def test_the_launches_of_a_submission_take_every_stream(lib, ctx, kinds, large):
 
 
 @pytest.mark.parametrize("n,threads,grid", [
-    (300, 32, 300),          # a warp per ROI, a ROI per block
-    (5_000, 128, 157),       # four lanes, 32 ROIs per block
+    (300, 128, 10),          # four lanes, 32 ROIs per block
+    (5_000, 128, 157),
     (100_000, 64, 4 * SMS),  # one thread, as many blocks as are resident (the fake's four per SM)
 ])
 def test_the_launches_without_allocation_go_by_their_own_kinds_rois(lib, n, threads, grid):
     """gmle_fit_mixed_device_noalloc's launches run one after another, so that a kind's
-    shape does not depend on what else the call holds."""
+    shape does not depend on how much else the call holds."""
     err = C.create_string_buffer(256)
-    shapes = []
-    for others in ([], [(1, 9, 200_000)], [(1, 9, 40)]):
-        gs = groups([(0, 11, n)] + others)
-        lib.fake_clear()
-        assert lib.gmle_fit_mixed_device_noalloc(gs, len(gs), None, None, None, 0, 0,
-                                                 C.c_void_p(999), err, 256) == 0, err.value
-        fits = [c for c in calls(lib, "launch") if c[1:3] != (1, 256)]  # (without the table writes)
-        assert len(fits) == len(gs) and all(c[0] == 999 for c in fits)
-        shapes.append(fits[0][1:3])
-    assert shapes == [(grid, threads)] * 3
+    for others in ([(1, 9, 200_000)], [(1, 9, 3_000)]):
+        shape = noalloc_shapes(lib, err, [(0, 11, n)] + others)[0]
+        assert shape == (grid, threads)
+
+
+def noalloc_shapes(lib, err, kinds):
+    gs = groups(kinds)
+    lib.fake_clear()
+    assert lib.gmle_fit_mixed_device_noalloc(gs, len(gs), None, None, None, 0, 0,
+                                             C.c_void_p(999), err, 256) == 0, err.value
+    fits = [c for c in calls(lib, "launch") if c[1:3] != (1, 256)]  # (without the table writes)
+    assert len(fits) == len(gs) and all(c[0] == 999 for c in fits)
+    return [c[1:3] for c in fits]
+
+
+@pytest.mark.parametrize("other,lanes", [(2_739, 32), (2_740, 4), (29_000, 4)])
+def test_small_kinds_take_the_lanes_of_the_entry_point_with_a_context(lib, ctx, other, lanes):
+    """A warp per ROI for all of a call below 20 ROIs per SM, else four lanes: as in
+    gmle_fit_mixed_device, so that the two give the same bits."""
+    kinds = [(0, 11, 300), (3, 15, other)]
+    mine = noalloc_shapes(lib, C.create_string_buffer(256), kinds)[0]
+    lib.fake_clear()
+    gs = groups(kinds)
+    assert lib.gmle_fit_mixed_device(ctx, gs, len(gs), C.c_void_p(999)) == 0
+    theirs = [c[1:3] for c in calls(lib, "launch")]
+    if lanes == 4:
+        assert mine == (10, 128) and mine in theirs
+    else:
+        assert mine == (300, 32) and all(t <= 128 for _, t in theirs)
 
 
 def get_tuning(lib, ctx, model, box, camera):
