@@ -335,7 +335,8 @@ __device__ __forceinline__ void walk_edge2(const Axis &a, EdgeWalk &w0, EdgeWalk
 // The entries of the R pixels from t0 on, their R + 1 edges in pairs: a row table
 // stands whole before the column loop, so its edges have no order to keep.  XYNB
 // 11x11 Poisson, 10^6 ROIs: 1631 -> 1622 us; XYNBS 13x13 sCMOS, 10^6: 3018 -> 2987;
-// astigmatic 15x15 Poisson, 300 000: 1192 -> 1181.
+// astigmatic 15x15 Poisson, 300 000: 1192 -> 1181 (with the erf argument's factor in the
+// polynomial, see EdgeWalk; 1669, 2993 and 1241 now).
 template <bool SIG, int R>
 __device__ __forceinline__ void edge_table(const Axis &a, int t0, float *psf, float *d1, float *d2,
                                            float *z1, float *zq)
@@ -1926,6 +1927,10 @@ __device__ __forceinline__ void fit_rois_r1(const KernelArgs &a, int64_t roi0, i
                 const float *col = pix + (j - 1) * BOX * PS;
                 float vv[LW];  // this column's variances, from tensor memory
                 if (SCMOS) tmem_ld<LW>(taddr + BOX * (j - 1), vv);
+                // an sCMOS ratio is summed by columns: one sum over all pixels rounds by
+                // more (XYNBS 13x13: 3.6e-7 of it, against 3.1e-7 so and with four lanes,
+                // whose sums are a quarter as long; 10^6 ROIs 2995 and 2992 us)
+                float part = 0.f;
                 float Q[NB][NB];
 #pragma unroll
                 for (int p = 0; p < NB; p++)
@@ -1936,8 +1941,10 @@ __device__ __forceinline__ void fit_rois_r1(const KernelArgs &a, int64_t roi0, i
                     const float d = col[t];
                     const float v = SCMOS ? vv[t] : 0.f;
                     const float mu = fmaf(npx, py[t], bg);
-                    final_pixel<SCMOS, SIG, NB>(d, v, mu, py[t], yd1[t], SIG ? ys1[t] : 0.f, llr, Q);
+                    final_pixel<SCMOS, SIG, NB>(d, v, mu, py[t], yd1[t], SIG ? ys1[t] : 0.f,
+                                                SCMOS ? part : llr, Q);
                 }
+                if (SCMOS) llr += part;
                 fisher_column<MODEL, P, NB>(Fh, Fl, Q, xp, xd1, xs1);
                 xp = nxp; xd1 = nxd1; xs1 = nxs1;
             }
