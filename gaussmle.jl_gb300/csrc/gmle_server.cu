@@ -53,10 +53,13 @@ constexpr int kRunStreams = 6;
 constexpr int kServerTableCap = 4096;  // groups (requests) per step and kind
 // Requests of this many ROIs, and of boxes up to 10 pixels, are fitted with one
 // thread per ROI, the others with four lanes: by the request's own size, so that
-// its results do not depend on the step it runs in.  One thread takes half the
+// its results do not depend on the step it runs in.  (None takes a warp per ROI: many
+// small requests make a step.)  One thread takes half the
 // work per ROI, but a larger box's fit a third longer (astigmatic 15x15 sCMOS: 129
 // us against 76) until a request fills the GPU by itself.
-// Line at 4 000 / 12 000 ROIs (us): 28 460 sCMOS ROIs in 7 requests 363 / 321,
+// The length of a block depends on model and box; the line, one count of ROIs, does not.
+// It is drawn for many small requests, and costs a few large ones:
+// line at 4 000 / 12 000 ROIs (us): 28 460 sCMOS ROIs in 7 requests 363 / 321,
 // 100 000 in 40 requests 745 / 714, in 10 requests 570 / 630 (with four lanes for
 // every box above 10: 350, 890, 790, before those were made faster).
 constexpr int64_t kLargeRequest = 12000;
